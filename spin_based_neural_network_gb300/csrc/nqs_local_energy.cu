@@ -2,13 +2,11 @@
 // nqs_local_energy* entry points.
 //
 // Fused estimator (RBM / complex RBM, any Marshall layers): one warp per
-// sample.  Each lane computes theta_h for its hidden units once, caches
-// log(2 cosh theta_h), and every connected configuration s' (single flip at u
-// or pair flip (u, v)) costs one O(M) update
-//     theta'_h = theta_h - 2 s_u W_hu [- 2 s_v W_hv]
-// plus M complex log-cosh evaluations and one warp butterfly, instead of the
-// upstream O(N M) recomputation per connected configuration
-// (src/nqs/nqs_gradient.c:24-30).  The same theta feeds the Jacobian row.
+// sample.  theta_h of the sample is formed once, and the amplitude ratio of a connected
+// configuration s' (single flip at u or pair flip (u, v)) is a product over the hidden units
+// of factors that need no transcendental, instead of the upstream O(N M) recomputation of
+// log 2 cosh per connected configuration (src/nqs/nqs_gradient.c:24-30).  The same theta
+// feeds the Jacobian row.
 #include <math.h>
 
 #include "nqs_amp.cuh"
@@ -207,146 +205,298 @@ __device__ void rbm_row_from_t(const DevAnsatz &a, uint64_t bits, int mode, doub
     }
 }
 
-template <int J, bool CPLX>
+// ---------------------------------------------------------------- FP64 product form
+// A flip of site u (and v) moves theta_h by -s_u D_h, D_h = 2 (W_hu - W_hv) for the pair flips
+// of the spin Hamiltonians (s_v = -s_u, or the ratio is not needed) and D_h = 2 W_hu for
+// single flips.  With r_h = exp(-2 theta_h) where Re theta_h >= 0 and exp(2 theta_h) where not,
+//   cosh(theta_h - s_u D_h) / cosh(theta_h) = (L + X r_h) / (1 + r_h),
+// L and X being exp(-s_u D_h) and exp(s_u D_h), exchanged where Re theta_h < 0.  |r_h| <= 1, so
+// no term cancels that does not cancel in cosh itself, and a connected configuration costs two
+// multiply-adds and a product per hidden unit (eight FP64 instructions, two for the real RBM)
+// where log 2 cosh of every unit cost about 200: this GPU issues an FP64 warp instruction per
+// 16 clocks and SM, and the estimator is bound by their number.  prod 1 / (1 + r_h) is one
+// factor per sample.
+//
+// Measured: kagome 3x3, complex RBM M = 54, 3001 configurations: 185 us and 12 us for the tables,
+// against 1999 us by logarithms; 4x4 Heisenberg, complex RBM M = 32, 1000 samples with Jacobian
+// rows: 45 + 12 against 339 us; 4x4 TFIM, RBM M = 16, 256 samples: 16 + 6 against 92 us.
+
+// Moves of a Hamiltonian: single flips of all sites (TFIM), else the pair flips of both bond groups.
+__host__ __device__ inline int num_moves(const DevHam &H) {
+    return H.kind == NQS_HAM_TFIM ? H.N : H.nb1 + H.nb2;
+}
+__device__ __forceinline__ void move_sites(const DevHam &H, int m, int &u, int &v) {
+    if (H.kind == NQS_HAM_TFIM) {
+        u = m;
+        v = -1;
+        return;
+    }
+    const int *b = m < H.nb1 ? H.b1 + 2 * m : H.b2 + 2 * (m - H.nb1);
+    u = b[0];
+    v = b[1];
+}
+
+// Flip tables, one warp per move: row m holds exp(D_h), exp(-D_h) of the hidden units (CPLX: re,
+// im each) and in column M the same of the visible biases.  range_ok[m] says that the products of
+// the row stay within the range of a double: sum_h |Re D_h| <= 350, and the factors are at most
+// 2 exp|Re D_h| (M <= 256), so nothing exceeds 2^256 e^350 < 1e230.
+constexpr double kFlipRange = 350.0;
+template <bool CPLX>
+__global__ void __launch_bounds__(128) k_flip_tables(DevAnsatz a, DevHam H, int nm, double *tab, int *range_ok) {
+    const int lane = threadIdx.x & 31, m = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (m >= nm) return;
+    constexpr int W = CPLX ? 4 : 2;
+    const int M = a.M;
+    const double *aR = a.p, *aI = a.p + crbm_pr(a);
+    int u, v;
+    move_sites(H, m, u, v);
+    double sum = 0.0;
+    for (int h = lane; h <= M; h += 32) {
+        double x = h < M ? a.wtr[(long)u * M + h] : aR[u], y = 0.0;
+        if (v >= 0) x -= h < M ? a.wtr[(long)v * M + h] : aR[v];
+        if (CPLX) {
+            y = h < M ? a.wti[(long)u * M + h] : aI[u];
+            if (v >= 0) y -= h < M ? a.wti[(long)v * M + h] : aI[v];
+        }
+        x *= 2.0;
+        y *= 2.0;
+        const double ep = exp(x), em = exp(-x);
+        double *t = tab + ((size_t)m * (M + 1) + h) * W;
+        if (CPLX) {
+            double sn, cs;
+            sincos(y, &sn, &cs);
+            t[0] = ep * cs;
+            t[1] = ep * sn;
+            t[2] = em * cs;
+            t[3] = -em * sn;
+        } else {
+            t[0] = ep;
+            t[1] = em;
+        }
+        sum += fabs(x);
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) range_ok[m] = sum <= kFlipRange;        // false for NaN too
+}
+
+// psi(s2) / psi(s) through the logarithms: the moves whose products could leave a double's range.
+__device__ __noinline__ void log_ratio(const DevAmp &A, uint64_t s, uint64_t s2, double &re, double &im) {
+    double l0, a0, l1, a1, sn, cs;
+    warp_amp_eval(A, s, l0, a0, nullptr);
+    warp_amp_eval(A, s2, l1, a1, nullptr);
+    const double mag = exp(l1 - l0);
+    sincos(a1 - a0, &sn, &cs);
+    re = mag * cs;
+    im = mag * sn;
+}
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+    return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
+}
+
+// Bytes of shared memory a warp of k_local_prod takes.
+static size_t local_prod_smem(int M, int nm) { return sizeof(double) * 2 * M + 32 + (size_t)(nm + 3) / 4 * 8; }
+
+// Local energies (and Jacobian rows) of the RBM / complex RBM, one warp per sample.  The warp
+// forms r_h with its lanes over the hidden units, then its 32 / L groups of L lanes take one
+// connected configuration each: a lane multiplies the factors of its J units (J L >= M) and the
+// group multiplies its lanes' products (log2 L steps; small L keeps that short, and L = 8, 16, 32
+// up to M = 64, 128, 256 bounds a lane's registers).  Lane k of a group keeps the product of the
+// group's k-th configuration, so visible factors, signs and couplings are done 32 configurations
+// at a time.
+template <int L, int J, bool CPLX>
 __global__ void __launch_bounds__(32 * kWarps)
-k_local_rbm(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, double *__restrict__ Er,
-            double *__restrict__ Ei, double *__restrict__ O, double *__restrict__ Oi, int grad_mode,
-            double *__restrict__ la_out) {
-    extern __shared__ double sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarps + warp;
+k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, double *__restrict__ Er,
+             double *__restrict__ Ei, double *__restrict__ O, double *__restrict__ Oi, int grad_mode,
+             const double *__restrict__ tab, const int *__restrict__ range_ok, int nm, int warp_bytes) {
+    extern __shared__ __align__(16) unsigned char smb[];
+    constexpr int W = CPLX ? 4 : 2, Q = (L * J + 31) / 32, GR = 32 / L;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sl = lane % L, sg = lane / L;
+    const int b = blockIdx.x * (blockDim.x >> 5) + warp;
     if (b >= B) return;
     const DevAnsatz &a = A.a;
     const int N = a.N, M = a.M;
-    const double *aR = a.p;
-    const double *aI = a.p + crbm_pr(a);
+    double *rs = (double *)(smb + (size_t)warp * warp_bytes);      // [2 M]: r, later tanh(theta)
+    uint32_t *negs = (uint32_t *)(rs + 2 * M);                      // [8]: Re theta_h < 0
+    unsigned short *list = (unsigned short *)(negs + 8);            // [nm]
     const uint64_t s = bits[b];
 
-    double thr[J], thi[J], lr[J], li[J];
+    double thr[Q], thi[Q];
+    double2 P = make_double2(1.0, 0.0);                             // prod_h (1 + r_h)
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const int h = lane + 32 * q;
+        thr[q] = thi[q] = 0.0;
+        if (h < M) {
+            double xr = a.p[N + h], xi = CPLX ? a.p[crbm_pr(a) + N + h] : 0.0;
+            for (int i = 0; i < N; i++) {
+                xr += sflip(a.wtr[(long)i * M + h], s, i);
+                if (CPLX) xi += sflip(a.wti[(long)i * M + h], s, i);
+            }
+            thr[q] = xr;
+            thi[q] = xi;
+            const double e = exp(-2.0 * fabs(xr)) + (xr - xr);      // NaN, not 0, for an infinite theta
+            if (CPLX) {
+                double sn, cs;
+                sincos(2.0 * xi, &sn, &cs);
+                const double2 r = make_double2(e * cs, xr < 0.0 ? e * sn : -(e * sn));
+                rs[2 * h] = r.x;
+                rs[2 * h + 1] = r.y;
+                P = cmul(P, make_double2(1.0 + r.x, r.y));
+            } else {
+                rs[h] = e;
+                P.x *= 1.0 + e;
+            }
+        }
+        const uint32_t neg = __ballot_sync(0xffffffffu, thr[q] < 0.0);
+        if (lane == 0) negs[q] = neg;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(0xffffffffu, P.x, o);
+        if (CPLX) P = cmul(P, make_double2(x, __shfl_xor_sync(0xffffffffu, P.y, o)));
+        else P.x *= x;
+    }
+    // 1 / P (scaled: |P| <= 2^256)
+    if (CPLX) {
+        const double big = fmax(fabs(P.x), fabs(P.y)), x = P.x / big, y = P.y / big, d = big * fma(x, x, y * y);
+        P = make_double2(x / d, -y / d);
+    } else {
+        P.x = 1.0 / P.x;
+    }
+
+    // connected configurations: the moves with antiparallel spins (all of them for single flips)
+    const bool tfim = H.kind == NQS_HAM_TFIM;
+    int n = 0, sum1 = 0, sum2 = 0, slow = 0;                        // sums of s_u s_v over the bond groups
+    for (int m0 = 0; m0 < nm; m0 += 32) {
+        const int m = m0 + lane;
+        int u = 0, v = -1;
+        if (m < nm) move_sites(H, m, u, v);
+        const int su = (int)((s >> u) & 1ull);
+        const bool anti = m < nm && (tfim || su != (int)((s >> v) & 1ull));
+        const bool ok = anti && range_ok[m] != 0;
+        const uint32_t am = __ballot_sync(0xffffffffu, anti);
+        if (!tfim) {
+            const uint32_t in = __ballot_sync(0xffffffffu, m < nm), g1 = __ballot_sync(0xffffffffu, m < H.nb1);
+            sum1 += __popc(g1) - 2 * __popc(am & g1);
+            sum2 += __popc(in & ~g1) - 2 * __popc(am & ~g1);
+        }
+        const uint32_t okm = __ballot_sync(0xffffffffu, ok);
+        if (ok) list[n + __popc(okm & ((1u << lane) - 1))] = (unsigned short)(m | (su << 15));
+        n += __popc(okm);
+        slow += __popc(am & ~okm);
+    }
+    if (tfim)
+        for (int m0 = 0; m0 < H.nb1; m0 += 32) {
+            const int k = m0 + lane;
+            const bool in = k < H.nb1;
+            const bool anti = in && (((s >> H.b1[2 * k]) ^ (s >> H.b1[2 * k + 1])) & 1ull);
+            sum1 += __popc(__ballot_sync(0xffffffffu, in)) - 2 * __popc(__ballot_sync(0xffffffffu, anti));
+        }
+    __syncwarp();
+    double rr[J], ri[J];
+    uint32_t neg = 0;
 #pragma unroll
     for (int j = 0; j < J; j++) {
-        int h = lane + 32 * j;
-        thr[j] = thi[j] = lr[j] = li[j] = 0.0;
+        const int h = sl + L * j;
+        rr[j] = ri[j] = 0.0;
         if (h < M) {
-            rbm_theta(a, s, h, thr[j], thi[j]);
-            if (CPLX) clogcosh(thr[j], thi[j], lr[j], li[j]);
-            else lr[j] = logcosh_r(thr[j]);
+            rr[j] = rs[CPLX ? 2 * h : h];
+            if (CPLX) ri[j] = rs[2 * h + 1];
+            neg |= ((negs[h >> 5] >> (h & 31)) & 1u) << j;
         }
     }
     const int par0 = marshall_count(A, s);
-
-    // psi(s') / psi(s) for s' = s with sites u (and v >= 0) flipped
-    auto ratio = [&](int u, int v, double &rre, double &rim) {
-        const double su = (double)spin_of(s, u);
-        const double sv = v >= 0 ? (double)spin_of(s, v) : 0.0;
-        double dla = 0.0, dar = 0.0;
+    const double c1 = tfim ? -H.Gamma : 0.5 * H.Jxy, c2 = 0.5 * H.J2;
+    double ore = 0.0, oim = 0.0;
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        double2 keep = make_double2(0.0, 0.0);
+        int km = 0;
+#pragma unroll 1
+        for (int k = 0; k < L && c0 + k * GR < n; k++) {
+            const int c = c0 + k * GR + sg;
+            double2 p = make_double2(1.0, 0.0);
+            int e = 0;
+            if (c < n) {
+                e = list[c];
+                const double *row = tab + (size_t)(e & 0x7fff) * (M + 1) * W;
+                const uint32_t sel = (e >> 15) ? ~neg : neg;        // leading factor exp(D) where set
 #pragma unroll
-        for (int j = 0; j < J; j++) {
-            int h = lane + 32 * j;
-            if (h < M) {
-                double xr = thr[j] - 2.0 * su * a.wtr[(long)u * M + h];
-                double xi = thi[j];
-                if (CPLX) xi -= 2.0 * su * a.wti[(long)u * M + h];
-                if (v >= 0) {
-                    xr -= 2.0 * sv * a.wtr[(long)v * M + h];
-                    if (CPLX) xi -= 2.0 * sv * a.wti[(long)v * M + h];
-                }
-                if (CPLX) {
-                    double l2, a2;
-                    clogcosh(xr, xi, l2, a2);
-                    dla += l2 - lr[j];
-                    dar += a2 - li[j];
-                } else {
-                    dla += logcosh_r(xr) - lr[j];
+                for (int j = 0; j < J; j++) {
+                    const int h = sl + L * j;
+                    if (h < M) {
+                        const bool q = (sel >> j) & 1u;
+                        if (CPLX) {
+                            const double2 *t = (const double2 *)(row + (size_t)h * W);
+                            const double2 Y = t[q ? 0 : 1], X = t[q ? 1 : 0];
+                            p = cmul(p, make_double2(fma(X.x, rr[j], fma(-X.y, ri[j], Y.x)),
+                                                     fma(X.x, ri[j], fma(X.y, rr[j], Y.y))));
+                        } else {
+                            const double2 t = *(const double2 *)(row + (size_t)h * W);
+                            p.x *= q ? fma(t.y, rr[j], t.x) : fma(t.x, rr[j], t.y);
+                        }
+                    }
                 }
             }
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) {
+                const double x = __shfl_xor_sync(0xffffffffu, p.x, o);
+                if (CPLX) p = cmul(p, make_double2(x, __shfl_xor_sync(0xffffffffu, p.y, o)));
+                else p.x *= x;
+            }
+            if (sl == k) {
+                keep = p;
+                km = e;
+            }
         }
-        dla = warp_sum(dla);
-        if (CPLX) dar = warp_sum(dar);
-        dla += -2.0 * su * aR[u];
-        if (CPLX) dar += -2.0 * su * aI[u];
-        uint64_t s2 = s ^ (1ull << u);
-        if (v >= 0) {
-            dla += -2.0 * sv * aR[v];
-            if (CPLX) dar += -2.0 * sv * aI[v];
-            s2 ^= 1ull << v;
+        const int c = c0 + sl * GR + sg;
+        if (c < n) {
+            const int m = km & 0x7fff;
+            const double *t = tab + ((size_t)m * (M + 1) + M) * W;
+            int u, v;
+            move_sites(H, m, u, v);
+            const uint64_t s2 = s ^ (1ull << u) ^ (v >= 0 ? 1ull << v : 0ull);
+            const double cf = m < H.nb1 || tfim ? c1 : c2;
+            const double sc = ((marshall_count(A, s2) - par0) & 1) ? -cf : cf;
+            const int q = (km >> 15) ? 0 : 1;                       // exp(-s_u D) of the visible biases
+            if (CPLX) {
+                const double2 w = cmul(cmul(keep, P), ((const double2 *)t)[q]);
+                ore = fma(sc, w.x, ore);
+                oim = fma(sc, w.y, oim);
+            } else {
+                ore = fma(sc, keep.x * P.x * t[q], ore);
+            }
         }
-        dar += kPi * (double)(marshall_count(A, s2) - par0);
-        double mag = exp(dla);
-        double sn, cs;
-        sincos(dar, &sn, &cs);
-        rre = mag * cs;
-        rim = mag * sn;
-    };
-
-    double e_re, e_im;
-    if (H.kind == NQS_HAM_TFIM) {                        // src/nqs/nqs_gradient.c:50-82
-        double diag = 0.0;
-        for (int k = 0; k < H.nb1; k++)
-            diag += -H.J * (double)(spin_of(s, H.b1[2 * k]) * spin_of(s, H.b1[2 * k + 1]));
-        double ore = 0.0, oim = 0.0;
-        for (int i = 0; i < N; i++) {
+    }
+    ore = warp_sum(ore);
+    if (CPLX) oim = warp_sum(oim);
+    if (slow > 0)                                                   // products out of range: by logarithms
+        for (int m = 0; m < nm; m++) {
+            int u, v;
+            move_sites(H, m, u, v);
+            if (range_ok[m] || (!tfim && (((s >> u) ^ (s >> v)) & 1ull) == 0)) continue;
             double r, q;
-            ratio(i, -1, r, q);
-            ore += -H.Gamma * r;
-            oim += -H.Gamma * q;
+            log_ratio(A, s, s ^ (1ull << u) ^ (v >= 0 ? 1ull << v : 0ull), r, q);
+            const double cf = m < H.nb1 || tfim ? c1 : c2;
+            ore += cf * r;
+            oim += cf * q;
         }
-        e_re = diag + ore;
-        e_im = oim;
-    } else {                                             // :87-139, :146-205, :374-445
-        double diag = 0.0, ore = 0.0, oim = 0.0;
-        for (int k = 0; k < H.nb1; k++) {
-            int u = H.b1[2 * k], v = H.b1[2 * k + 1];
-            int su = spin_of(s, u), sv = spin_of(s, v);
-            diag += 0.25 * H.Jz * (double)(su * sv);
-            if (su != sv) {
-                double r, q;
-                ratio(u, v, r, q);
-                ore += 0.5 * H.Jxy * r;
-                oim += 0.5 * H.Jxy * q;
-            }
-        }
-        e_re = diag + ore;
-        e_im = oim;
-        if (H.nb2 > 0) {
-            double d2 = 0.0, r2 = 0.0, i2 = 0.0;
-            for (int k = 0; k < H.nb2; k++) {
-                int u = H.b2[2 * k], v = H.b2[2 * k + 1];
-                int su = spin_of(s, u), sv = spin_of(s, v);
-                d2 += 0.25 * H.J2 * (double)(su * sv);
-                if (su != sv) {
-                    double r, q;
-                    ratio(u, v, r, q);
-                    r2 += 0.5 * H.J2 * r;
-                    i2 += 0.5 * H.J2 * q;
-                }
-            }
-            e_re = e_re + d2 + r2;
-            e_im = e_im + i2;
-        }
-    }
     if (lane == 0) {
-        if (Er) Er[b] = e_re;
-        if (Ei) Ei[b] = e_im;
-    }
-    if (la_out) {
-        double sr = 0.0;
-#pragma unroll
-        for (int j = 0; j < J; j++) sr += lr[j];
-        double vr, vi;
-        warp_visible(a, s, vr, vi);
-        sr = vr + warp_sum(sr);
-        if (lane == 0) la_out[b] = sr;
+        double diag = tfim ? -H.J * (double)sum1 : 0.25 * H.Jz * (double)sum1;
+        if (H.nb2 > 0) diag += 0.25 * H.J2 * (double)sum2;
+        if (Er) Er[b] = diag + ore;
+        if (Ei) Ei[b] = oim;
     }
     if (grad_mode) {
-        double *tr = sm + warp * 2 * M, *ti = tr + M;
+        __syncwarp();
+        double *tr = rs, *ti = rs + M;
 #pragma unroll
-        for (int j = 0; j < J; j++) {
-            int h = lane + 32 * j;
+        for (int q = 0; q < Q; q++) {
+            const int h = lane + 32 * q;
             if (h < M) {
-                if (CPLX) ctanh_d(thr[j], thi[j], tr[h], ti[h]);
+                if (CPLX) ctanh_d(thr[q], thi[q], tr[h], ti[h]);
                 else {
-                    tr[h] = tanh(thr[j]);
+                    tr[h] = tanh(thr[q]);
                     ti[h] = 0.0;
                 }
             }
@@ -357,7 +507,7 @@ k_local_rbm(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, double
 }
 
 // ---------------------------------------------------------------- FP32 estimator
-// Mixed-precision variant of k_local_rbm for the RBM / cRBM.  A flip of site u
+// Mixed-precision variant of k_local_prod for the RBM / cRBM.  A flip of site u
 // (and v) moves theta_h by delta_h = 2 s_u W_hu (+ 2 s_v W_hv), and
 //   cosh(theta_h - delta_h) / cosh(theta_h) = cosh(delta_h) - tanh(theta_h) sinh(delta_h),
 // so with t_h = tanh(theta_h) once per sample and cosh / sinh(2 W) tabulated
@@ -769,16 +919,47 @@ static bool launch_mlp32(const DevAmp &A, const DevHam &H, const uint64_t *bits,
 }
 
 template <int J, bool C>
-static void launch_rbm(const DevAmp &A, const DevHam &H, const uint64_t *bits, int B, double *Er,
-                       double *Ei, double *O, double *Oi, int gm, bool f32) {
+static void launch_rbm32(const DevAmp &A, const DevHam &H, const uint64_t *bits, int B, double *Er,
+                         double *Ei, double *O, double *Oi, int gm) {
     size_t smem = gm ? sizeof(double) * 2 * A.a.M * kWarps : 0;
-    if (f32)
-        k_local_rbm32<J, C><<<(B + kWarps - 1) / kWarps, 32 * kWarps, smem, ctx().stream>>>(A, H, bits, B, Er,
-                                                                                          Ei, O, Oi, gm);
-    else
-        k_local_rbm<J, C><<<(B + kWarps - 1) / kWarps, 32 * kWarps, smem, ctx().stream>>>(A, H, bits, B, Er,
-                                                                                        Ei, O, Oi, gm,
-                                                                                        nullptr);
+    k_local_rbm32<J, C><<<(B + kWarps - 1) / kWarps, 32 * kWarps, smem, ctx().stream>>>(A, H, bits, B, Er,
+                                                                                      Ei, O, Oi, gm);
+}
+
+// FP64 estimator: the flip tables of this call's parameters and moves, then the samples.
+static DevBuf<double> g_flip;
+static DevBuf<int> g_flip_ok;
+
+template <bool C>
+static bool launch_prod(const DevAmp &A, const DevHam &H, const uint64_t *bits, int B, double *Er, double *Ei,
+                        double *O, double *Oi, int gm) {
+    const int nm = num_moves(H), M = A.a.M;
+    if (!g_flip.ensure((size_t)(nm + 1) * (M + 1) * (C ? 4 : 2)) || !g_flip_ok.ensure((size_t)nm + 1)) return false;
+    cudaStream_t st = ctx().stream;
+    {
+        NQS_LAUNCH("flip_tables");
+        k_flip_tables<C><<<(nm + 3) / 4, 128, 0, st>>>(A.a, H, nm, g_flip.p, g_flip_ok.p);
+    }
+    // warps per block: one while the samples fill less than two blocks per SM, so that a small
+    // batch spreads over the SMs (each has its own FP64 pipe)
+    const int wpb = B <= 2 * ctx().sm_count ? 1 : B <= 4 * ctx().sm_count ? 2 : kWarps;
+    const int wb = (int)local_prod_smem(M, nm);
+    NQS_LAUNCH("local_estimator");
+#define NQS_CASE(LL, JJ)                                                                                     \
+    case JJ:                                                                                                 \
+        k_local_prod<LL, JJ, C><<<(B + wpb - 1) / wpb, 32 * wpb, (size_t)wb * wpb, st>>>(                    \
+            A, H, bits, B, Er, Ei, O, Oi, gm, g_flip.p, g_flip_ok.p, nm, wb);                                \
+        break;
+    // units per lane rounded up to an even count: the units past M cost a skipped branch
+    if (M <= 64) {
+        switch ((M + 15) / 16 * 2) { NQS_CASE(8, 2) NQS_CASE(8, 4) NQS_CASE(8, 6) NQS_CASE(8, 8) }
+    } else if (M <= 128) {
+        switch ((M + 31) / 32 * 2) { NQS_CASE(16, 6) NQS_CASE(16, 8) }
+    } else {
+        switch ((M + 63) / 64 * 2) { NQS_CASE(32, 6) NQS_CASE(32, 8) }
+    }
+#undef NQS_CASE
+    return NQS_CUDA(cudaGetLastError());
 }
 
 bool fp32_capable(const DevAmp &A) {
@@ -808,20 +989,23 @@ bool launch_local_estimator(const DevAmp &A, const DevHam &H, const uint64_t *bi
     }
     const bool fused = A.G == 0 && (A.a.kind == KIND_RBM || A.a.kind == KIND_CRBM);
     if (fused) {
-        int J = (A.a.M + 31) / 32;
-        bool c = A.a.kind == KIND_CRBM;
-        const bool f32 = fp32 && fp32_capable(A);
-        NQS_LAUNCH(f32 ? "local_estimator_fp32" : "local_estimator");
+        const int J = (A.a.M + 31) / 32;
+        const bool c = A.a.kind == KIND_CRBM;
+        if (A.a.M > 32 * kMaxJ) {
+            set_error("hidden width %d unsupported", A.a.M);
+            return false;
+        }
+        if (!(fp32 && fp32_capable(A)))
+            return c ? launch_prod<true>(A, H, bits, B, Er, Ei, O, Oi, grad_mode)
+                     : launch_prod<false>(A, H, bits, B, Er, Ei, O, Oi, grad_mode);
+        NQS_LAUNCH("local_estimator_fp32");
 #define NQS_CASE(JJ)                                                                   \
     case JJ:                                                                           \
-        if (c) launch_rbm<JJ, true>(A, H, bits, B, Er, Ei, O, Oi, grad_mode, f32);     \
-        else launch_rbm<JJ, false>(A, H, bits, B, Er, Ei, O, Oi, grad_mode, f32);      \
+        if (c) launch_rbm32<JJ, true>(A, H, bits, B, Er, Ei, O, Oi, grad_mode);        \
+        else launch_rbm32<JJ, false>(A, H, bits, B, Er, Ei, O, Oi, grad_mode);         \
         break;
         switch (J) {
             NQS_CASE(1) NQS_CASE(2) NQS_CASE(3) NQS_CASE(4) NQS_CASE(5) NQS_CASE(6) NQS_CASE(7) NQS_CASE(8)
-            default:
-                set_error("hidden width %d unsupported", A.a.M);
-                return false;
         }
 #undef NQS_CASE
         return NQS_CUDA(cudaGetLastError());
