@@ -309,8 +309,8 @@ int nqs_gpu_gram_tc(const double *O_host, int num_samples, long num_params, int 
 int nqs_gpu_ess(const double *energies, int num_samples, int num_chains, double *out_tau, double *out_ess);
 
 /* Test hook: the number of polls a grid-wide barrier of the cooperative solve kernels
- * (mixed MinSR factor / refinement, CG-SR, batches) waits before it gives up; 0 restores
- * the default (2^24).  A barrier that gives up raises the kernel's error word, every CTA
+ * (FP64 MinSR factor, mixed MinSR factor / refinement, CG-SR, batches) waits before it
+ * gives up; 0 restores the default (2^24).  A barrier that gives up raises the kernel's error word, every CTA
  * leaves at its next barrier (releasing its tensor memory), and the step returns -1 with
  * "grid barrier timed out" in nqs_gpu_last_error(); the next call starts from cleared
  * barrier and error words. */

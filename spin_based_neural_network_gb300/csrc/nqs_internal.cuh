@@ -220,6 +220,10 @@ bool launch_symproj_gradient(const DevAmp &A, const uint64_t *bits, int B, doubl
 bool launch_symproj_gradient_complex(const DevAmp &A, const uint64_t *bits, int B, double *O, double *Oi);
 bool launch_bits_to_spins(const uint64_t *bits, int B, int N, int *out);
 
+// FP64 Cholesky and solve T y = b (nqs_chol64.cu).
+bool chol64_factor_solve(double *T, int n, const double *b, double *y, int *status, int **err_out);
+bool chol64_set_barrier_budget(unsigned v, cudaStream_t st);
+
 // CG-SR solve (S + eps I) d = F in one cooperative launch (upstream cg_solve
 // semantics); writes d, scal[S_RS, S_RS0, S_PAP], status[I_DONE, I_ITERS, I_CONV].
 bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double *gm, double eps, double tol,

@@ -25,6 +25,7 @@
 #include <math.h>
 
 #include "nqs_amp.cuh"
+#include "nqs_grid.cuh"
 #include "nqs_tc.cuh"
 
 namespace nqs {
@@ -335,46 +336,6 @@ __device__ __forceinline__ unsigned long long gtimer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
-}
-
-// Polls a grid barrier waits before it gives up (raising *err = 2).  A device variable so
-// that graph replays read the current value; nqs_gpu_set_barrier_budget() lowers it for
-// the tests of the timeout path.
-__device__ unsigned g_barrier_budget = 1u << 24;
-
-// A monotonic arrival counter (bar[0], cleared at every launch): the arrival that returns
-// old belongs to barrier instance old / count, which is passed once the counter reaches
-// (old / count + 1) * count, so no reset and no second word is needed (a CTA can only
-// arrive at the next instance after all arrivals of this one).  Ordering: the block
-// barrier, then an acq_rel fence at GPU scope around the relaxed atomic and the polls.
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned count) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned budget = *(volatile unsigned *)&g_barrier_budget;
-        unsigned old;
-        asm volatile("fence.acq_rel.gpu;\n\tatom.relaxed.gpu.global.add.u32 %0, [%1], 1;"
-                     : "=r"(old) : "l"(bar) : "memory");
-        const unsigned target = (old / count + 1u) * count;
-        uint32_t it = 0;
-        for (;;) {
-            unsigned cur;
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(bar) : "memory");
-            if ((int)(cur - target) >= 0) break;
-            if (++it > budget) {
-                atomicExch(err, 2);
-                break;
-            }
-            if ((it & 31) == 0) {                       // the error word every 32nd poll only
-                if (*((volatile int *)err)) break;
-                if (it > 256) __nanosleep(32);
-            }
-        }
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        s_ok = *((volatile int *)err) == 0;
-    }
-    __syncthreads();
-    return s_ok != 0;                                 // one answer for the whole CTA
 }
 
 // Factor the 128 x 128 block in S (rows >= bs padded with the identity) in four
@@ -2874,7 +2835,7 @@ int nqs_gpu_set_barrier_budget(unsigned polls) {
     const unsigned v = polls ? polls : (1u << 24);
     cudaStream_t st = ctx().stream;
     return NQS_CUDA(cudaMemcpyToSymbolAsync(g_barrier_budget, &v, sizeof(v), 0, cudaMemcpyHostToDevice, st)) &&
-                   NQS_CUDA(cudaStreamSynchronize(st))
+                   NQS_CUDA(cudaStreamSynchronize(st)) && chol64_set_barrier_budget(v, st)
                ? 0
                : -1;
 }

@@ -7,9 +7,8 @@
 //   -> energy statistics (compensated) and eps_i = E_i - <E>
 //   -> column means <O_k>, centring O_c = O - <O>
 //   -> T = O_c O_c^T / N_s + shift I (lower triangle, 64x64 tiles)
-//   -> blocked right-looking Cholesky (32-wide panels: diagonal-block factor,
-//      panel triangular solve, trailing SYRK update), status word on device
-//   -> forward / backward blocked triangular solves
+//   -> blocked right-looking Cholesky and the triangular solves in one cooperative
+//      launch (nqs_chol64.cu), status word on device
 //   -> delta = O_c^T y / N_s, theta -= lr delta, ||delta||.
 #include <algorithm>
 #include <cuda.h>
@@ -24,7 +23,7 @@ bool sampler_produce(Sampler *s, int n, uint64_t **d_out);
 
 // ---------------------------------------------------------------- workspace
 struct Workspace {
-    DevBuf<double> E, Ei, eps, O, gm, T, T0, y, z, delta, scal, F, r, p, Ap, u, part, y64, d64, es;
+    DevBuf<double> E, Ei, eps, O, gm, T, T0, y, delta, scal, F, r, p, Ap, u, part, y64, d64, es;
     DevBuf<double> Oi, gm2, F2, scal2, eps2, es2;     // holomorphic SR: imaginary halves
     DevBuf<double> la, ar, la_ref, ar_ref, aug;       // excited-state SR: amplitude ratios, augmented means
     DevBuf<double> theta0, kacc;                      // Heun tVMC: parameter snapshot, averaged slope
@@ -596,29 +595,6 @@ __global__ void __launch_bounds__(256) k_syrk_update(double *A, int n, int k0, i
         }
 }
 
-static bool cholesky_fp64(double *T, int n, int *status) {
-    cudaStream_t st = ctx().stream;
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        int kb = n - k0 < NB ? n - k0 : NB;
-        {
-            NQS_LAUNCH("chol_diag");
-            k_potrf_diag<<<1, dim3(32, 32), 0, st>>>(T, n, k0, kb, status);
-        }
-        int k1 = k0 + kb, rest = n - k1;
-        if (rest <= 0) break;
-        {
-            NQS_LAUNCH("chol_panel");
-            k_trsm_panel<<<(rest + 127) / 128, 128, 0, st>>>(T, n, k0, kb, kb, k1, status, 0);
-        }
-        int nt = (rest + TG - 1) / TG;
-        {
-            NQS_LAUNCH("chol_syrk");
-            k_syrk_update<<<nt * (nt + 1) / 2, 256, 0, st>>>(T, n, k0, kb, k1, status);
-        }
-    }
-    return NQS_CUDA(cudaGetLastError());
-}
-
 // The upstream retry (src/nqs/nqs_optimizer.c:1156-1160) re-factors the matrix
 // as the failed column-by-column factorisation left it: columns c < j hold L
 // (every row), columns >= j hold the original T.  Rebuild exactly that state
@@ -683,24 +659,17 @@ __global__ void k_trsv_bwd(const double *__restrict__ L, int n, int k0, int kb, 
     }
 }
 
-static bool cholesky_solve(const double *L, int n, const double *b, double *z, double *y) {
+// FP64 factor and solve T y = b; *fail receives the first failing column (-1: solved).
+static bool factor_solve_fp64(double *T, int n, const double *b, double *y, int *status, int *fail) {
     cudaStream_t st = ctx().stream;
-    if (!NQS_CUDA(cudaMemcpyAsync(z, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st))) return false;
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        int kb = n - k0 < NB ? n - k0 : NB;
-        int rest = n - k0 - kb;
-        NQS_LAUNCH("trsv_fwd");
-        k_trsv_fwd<<<rest > 0 ? (rest + 127) / 128 : 1, 128, 0, st>>>(L, n, k0, kb, z, y);
-    }
-    // y now holds the forward solution; reuse it as the right-hand side
-    if (!NQS_CUDA(cudaMemcpyAsync(z, y, sizeof(double) * n, cudaMemcpyDeviceToDevice, st))) return false;
-    int last = ((n - 1) / NB) * NB;
-    for (int k0 = last; k0 >= 0; k0 -= NB) {
-        int kb = n - k0 < NB ? n - k0 : NB;
-        NQS_LAUNCH("trsv_bwd");
-        k_trsv_bwd<<<k0 > 0 ? (k0 + 127) / 128 : 1, 128, 0, st>>>(L, n, k0, kb, z, y);
-    }
-    return NQS_CUDA(cudaGetLastError());
+    int *derr = nullptr, herr = 0;
+    if (!chol64_factor_solve(T, n, b, y, status, &derr) ||
+        !NQS_CUDA(cudaMemcpyAsync(fail, status + I_FAIL, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
+        !NQS_CUDA(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
+        !NQS_CUDA(cudaStreamSynchronize(st)))
+        return false;
+    if (herr) set_error("FP64 Cholesky: grid barrier timed out");
+    return herr == 0;
 }
 
 // ---------------------------------------------------------------- update
@@ -917,18 +886,15 @@ int minsr_fp64_solve(const double *O, const double *eps, int Ns, long P, double 
     Context &c = ctx();
     cudaStream_t st = c.stream;
     *conv = 0;
-    if (!w.T.ensure((size_t)Ns * Ns) || !w.z.ensure(Ns) || !w.status.ensure(16)) return -1;
+    if (!w.T.ensure((size_t)Ns * Ns) || !w.status.ensure(16)) return -1;
     int nt = (Ns + TG - 1) / TG;
     NQS_CUDA(cudaMemsetAsync(w.status.p, 0xff, sizeof(int) * 16, st));
     {
         NQS_LAUNCH("gram_fp64");
         k_gram_fp64<<<nt * (nt + 1) / 2, 256, 0, st>>>(O, Ns, P, 1.0 / (double)Ns, shift, w.T.p);
     }
-    if (!cholesky_fp64(w.T.p, Ns, w.status.p)) return -1;
     int fail = -1;
-    if (!NQS_CUDA(cudaMemcpyAsync(&fail, w.status.p + I_FAIL, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
-        !NQS_CUDA(cudaStreamSynchronize(st)))
-        return -1;
+    if (!factor_solve_fp64(w.T.p, Ns, eps, y_out, w.status.p, &fail)) return -1;
     step_stats().chol_fail_col = fail;
     step_stats().chol_retry = 0;
     int fail2 = -1;
@@ -951,13 +917,9 @@ int minsr_fp64_solve(const double *O, const double *eps, int Ns, long P, double 
             k_quirk_restore<<<c.sm_count * 8, 256, 0, st>>>(w.T.p, w.T0.p, Ns, fail);
         }
         NQS_CUDA(cudaMemsetAsync(w.status.p + I_FAIL, 0xff, sizeof(int), st));
-        if (!cholesky_fp64(w.T.p, Ns, w.status.p)) return -1;
-        if (!NQS_CUDA(cudaMemcpyAsync(&fail2, w.status.p + I_FAIL, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
-            !NQS_CUDA(cudaStreamSynchronize(st)))
-            return -1;
+        if (!factor_solve_fp64(w.T.p, Ns, eps, y_out, w.status.p, &fail2)) return -1;
     }
     if (fail2 < 0) {
-        if (!cholesky_solve(w.T.p, Ns, eps, w.z.p, y_out)) return -1;
         *conv = 1;
     } else {
         fprintf(stderr, "nqs_sr_step_minsr: Cholesky breakdown after retry; increase "
@@ -1073,7 +1035,7 @@ int minsr_fp64_params(const double *O, const double *eps, int Ns, long P, double
     Workspace &w = g_ws;
     cudaStream_t st = ctx().stream;
     *conv = 0;
-    if (!w.z.ensure(P) || !w.r.ensure(P) || !w.status.ensure(16)) return -1;
+    if (!w.r.ensure(P) || !w.status.ensure(16)) return -1;
     // right-hand side b = O_c^T eps / N_s
     if (!enqueue_col_dot(O, Ns, P, eps, 1.0 / (double)Ns, w.r.p)) return -1;
     int fail = -1;
@@ -1081,10 +1043,7 @@ int minsr_fp64_params(const double *O, const double *eps, int Ns, long P, double
     for (int attempt = 0; attempt < 2; attempt++) {
         if (!gram_cols(O, Ns, P, shift + (attempt ? 1e-6 : 0.0))) return -1;
         NQS_CUDA(cudaMemsetAsync(w.status.p, 0xff, sizeof(int) * 16, st));
-        if (!cholesky_fp64(w.T.p, (int)P, w.status.p)) return -1;
-        if (!NQS_CUDA(cudaMemcpyAsync(&fail, w.status.p + I_FAIL, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
-            !NQS_CUDA(cudaStreamSynchronize(st)))
-            return -1;
+        if (!factor_solve_fp64(w.T.p, (int)P, w.r.p, delta, w.status.p, &fail)) return -1;
         if (attempt == 0) step_stats().chol_fail_col = fail;
         if (fail < 0) break;
         step_stats().chol_retry = 1;
@@ -1094,7 +1053,6 @@ int minsr_fp64_params(const double *O, const double *eps, int Ns, long P, double
                         "sr_diag_shift or num_samples. Update set to 0.\n");
         return NQS_CUDA(cudaMemsetAsync(delta, 0, sizeof(double) * P, st)) ? 0 : -1;
     }
-    if (!cholesky_solve(w.T.p, (int)P, w.r.p, w.z.p, delta)) return -1;
     *conv = 1;
     return 0;
 }
@@ -1211,7 +1169,7 @@ static int sr_step_impl(const StepIn &in, nqs_sr_step_info_t *info, double *out_
     if (in.minsr == 1 && fp32est && c.opts.mixed_check) {
         // reference for the check: the FP64 estimator, statistics and FP64
         // MinSR solve on the same samples
-        if (!w.T.ensure((size_t)Ns * Ns) || !w.y.ensure(Ns) || !w.z.ensure(Ns) || !w.y64.ensure(Ns) ||
+        if (!w.T.ensure((size_t)Ns * Ns) || !w.y.ensure(Ns) || !w.y64.ensure(Ns) ||
             !w.d64.ensure(P))
             return -1;
         if (!launch_local_estimator(A, H, bits, Ns, w.E.p, w.Ei.p, w.O.p, nullptr, 1, false)) return -1;
@@ -1273,7 +1231,7 @@ static int sr_step_impl(const StepIn &in, nqs_sr_step_info_t *info, double *out_
     int converged = 0, cg_iters = 0;
     bool applied = false;             // update and derived tables already enqueued
     if (in.minsr == 1 || hm) {
-        if (!w.T.ensure((size_t)rows * rows) || !w.y.ensure(rows) || !w.z.ensure(rows)) return -1;
+        if (!w.T.ensure((size_t)rows * rows) || !w.y.ensure(rows)) return -1;
         {
             NQS_LAUNCH("col_mean");
             if (!col_stats(w.O.p, Ns, P, nullptr, w.scal.p, w.gm.p, nullptr)) return -1;
