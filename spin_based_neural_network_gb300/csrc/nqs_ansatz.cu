@@ -311,10 +311,11 @@ struct PermEntry {
     std::vector<double> chars;
     DevBuf<int> d_perm;
     DevBuf<double> d_chars;
+    int bijective = 0;               // every row is a permutation of the sites
 };
 static std::map<const void *, PermEntry *> g_perm_cache;
 
-static bool stage_perm(const nqs_symproj_wrapper_t *w, const int **dp, const double **dc) {
+static bool stage_perm(const nqs_symproj_wrapper_t *w, const int **dp, const double **dc, int *bijective) {
     size_t np = (size_t)w->num_group_elements * w->num_sites;
     PermEntry *&e = g_perm_cache[(const void *)w->perm];
     if (!e) e = new PermEntry();
@@ -327,6 +328,12 @@ static bool stage_perm(const nqs_symproj_wrapper_t *w, const int **dp, const dou
                 set_error("symproj permutation entry %d out of range", w->perm[k]);
                 return false;
             }
+        e->bijective = 1;
+        for (size_t g = 0; g < np; g += w->num_sites) {
+            uint64_t seen = 0;
+            for (int i = 0; i < w->num_sites; i++) seen |= 1ull << w->perm[g + i];
+            if (__builtin_popcountll(seen) != w->num_sites) e->bijective = 0;
+        }
         e->perm.assign(w->perm, w->perm + np);
         e->chars.assign(w->characters, w->characters + w->num_group_elements);
         if (!e->d_perm.ensure(np) || !e->d_chars.ensure((size_t)w->num_group_elements)) return false;
@@ -338,6 +345,7 @@ static bool stage_perm(const nqs_symproj_wrapper_t *w, const int **dp, const dou
     }
     *dp = e->d_perm.p;
     *dc = e->d_chars.p;
+    *bijective = e->bijective;
     return true;
 }
 
@@ -454,7 +462,7 @@ bool build_amp(nqs_log_amp_fn_t fn, void *user, int num_sites, DevAmp *out, Ansa
                 return false;
             }
             out->G = w->num_group_elements;
-            if (!stage_perm(w, &out->perm, &out->chars)) return false;
+            if (!stage_perm(w, &out->perm, &out->chars, &out->perm_bijective)) return false;
         }
     }
     if (outer_tmp > 3 || inner_tmp > 3) {
@@ -493,6 +501,7 @@ __global__ void k_log_amp(DevAmp A, const uint64_t *__restrict__ bits, int B, do
 }
 
 bool launch_log_amp(const DevAmp &A, const uint64_t *bits, int B, double *la, double *ar) {
+    if (sym_log_amp_capable(A)) return launch_sym_log_amp(A, bits, B, la, ar);
     size_t smem = sizeof(double) * (size_t)scratch_per_warp(A.a) * kWarpsPerBlock;
     NQS_LAUNCH("log_amp");
     k_log_amp<<<(B + kWarpsPerBlock - 1) / kWarpsPerBlock, 32 * kWarpsPerBlock, smem, ctx().stream>>>(
@@ -830,6 +839,7 @@ bool launch_symproj_gradient_complex(const DevAmp &A, const uint64_t *bits, int 
         set_error("complex symmetry-projected gradient: MF, RBM and complex RBM base ansatze only");
         return false;
     }
+    if (sym_gradient_capable(A)) return launch_sym_gradient(A, bits, B, 2, O, Oi);
     if (!g_symw.ensure((size_t)B * 2 * A.G)) return false;
     size_t smem = sizeof(double) * (size_t)scratch_per_warp(A.a) * kWarpsPerBlock;
     NQS_LAUNCH("symproj_gradient_complex");
@@ -839,6 +849,7 @@ bool launch_symproj_gradient_complex(const DevAmp &A, const uint64_t *bits, int 
 }
 
 bool launch_symproj_gradient(const DevAmp &A, const uint64_t *bits, int B, double *O) {
+    if (sym_gradient_capable(A)) return launch_sym_gradient(A, bits, B, 1, O, nullptr);
     if (!g_symw.ensure((size_t)B * 2 * A.G)) return false;
     size_t smem = sizeof(double) * (size_t)scratch_per_warp(A.a) * kWarpsPerBlock;
     NQS_LAUNCH("symproj_gradient");

@@ -161,6 +161,7 @@ struct DevAmp {
     int G;                       // symmetry projection group size, 0 = none
     const int *perm;             // [G][N] device
     const double *chars;         // [G] device
+    int perm_bijective;          // every row of perm is a permutation of the sites
     int n_inner;                 // Marshall layers inside the projection
     uint64_t inner_mask[3];
 };
@@ -214,6 +215,15 @@ bool fp32_mlp_capable(const DevAmp &A);    // MLP with width <= 128 and FP32 tab
 bool launch_gradient(const DevAnsatz &a, const uint64_t *bits, int B, int mode, double *O, double *Oi);
 bool launch_symproj_gradient(const DevAmp &A, const uint64_t *bits, int B, double *O);
 bool launch_symproj_gradient_complex(const DevAmp &A, const uint64_t *bits, int B, double *O, double *Oi);
+// symmetry-projected RBM / complex RBM programs (nqs_symproj.cu); *done (device) = 0 leaves the
+// energies to the generic kernel
+bool sym_log_amp_capable(const DevAmp &A);
+bool launch_sym_log_amp(const DevAmp &A, const uint64_t *bits, int B, double *la, double *ar);
+bool sym_gradient_capable(const DevAmp &A);
+bool launch_sym_gradient(const DevAmp &A, const uint64_t *bits, int B, int mode, double *O, double *Oi);
+bool sym_energy_capable(const DevAmp &A, const DevHam &H);
+bool launch_sym_energy(const DevAmp &A, const DevHam &H, const uint64_t *bits, int B, double *Er, double *Ei,
+                       int **done);
 bool launch_bits_to_spins(const uint64_t *bits, int B, int N, int *out);
 
 // FP64 Cholesky and solve T y = b (nqs_chol64.cu).

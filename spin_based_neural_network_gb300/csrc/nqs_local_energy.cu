@@ -689,7 +689,8 @@ k_local_rbm32(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doub
 // configuration is evaluated from scratch, as upstream does.
 __global__ void __launch_bounds__(32 * kWarps)
 k_local_generic(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, double *Er, double *Ei,
-                double *la_out) {
+                const int *done) {
+    if (done && *done) return;                             // the projected product form has run
     extern __shared__ double sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * kWarps + warp;
@@ -756,7 +757,6 @@ k_local_generic(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, do
     if (lane == 0) {
         if (Er) Er[b] = e_re;
         if (Ei) Ei[b] = e_im;
-        if (la_out) la_out[b] = la0;
     }
 }
 
@@ -1012,9 +1012,14 @@ bool launch_local_estimator(const DevAmp &A, const DevHam &H, const uint64_t *bi
     }
     {
         size_t smem = sizeof(double) * 4 * (A.a.M ? A.a.M : 1) * kWarps;
+        int *done = nullptr;
+        // symmetry projections of the RBM / complex RBM by permutations (a map that is not one to one
+        // flips several sites of g s per flip of s)
+        if (sym_energy_capable(A, H) && A.perm_bijective && !launch_sym_energy(A, H, bits, B, Er, Ei, &done))
+            return false;
         NQS_LAUNCH("local_generic");
         k_local_generic<<<(B + kWarps - 1) / kWarps, 32 * kWarps, smem, ctx().stream>>>(A, H, bits, B, Er,
-                                                                                      Ei, nullptr);
+                                                                                      Ei, done);
         if (!NQS_CUDA(cudaGetLastError())) return false;
     }
     if (grad_mode) {
