@@ -2646,6 +2646,191 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_sr(CgArgs a) {
     }
 }
 
+// CG-SR for systems whose Jacobian fits the SMs' shared memory: CTA b keeps rows
+// [b R, b R + R) of O (and O2) there for the whole solve, and all CTAs carry p, r (and CTA 0 d) in
+// registers, E entries a thread, computed alike by every CTA.  An iteration is
+//   u_i = O_i p for the CTA's rows and their column sums sum_i O_ik u_i -> upart[b]   | grid barrier
+//   columns dealt to the CTAs: A p from the G partials and <u>                         | grid barrier
+//   p.Ap, the updates and r.r in every CTA,
+// two grid barriers where k_cg_sr has five and no pass over O outside shared memory.
+// What bounds it: at 256 x 288 the two barriers and the chains of dependent FP64 operations of the
+// dots (64 clocks an operation); at 1024 x 1688 complex the FP64 pipes (14 MFMA an iteration).
+// Measured per iteration: 256 x 288: 11 us (39 by k_cg_sr), 1024 x 288: 12 (61), 1024 x
+// 1688 holomorphic: 31 (61).
+constexpr int CG_MAX_P = 8 * PS_THREADS;
+
+// block sum of v, the same value in every thread and every CTA
+__device__ __forceinline__ double cg_block_sum(double v, double *red) {
+    v = warp_sum(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[threadIdx.x & (PS_THREADS / 32 - 1)];
+#pragma unroll
+    for (int o = PS_THREADS / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <int E, bool TWO>
+__global__ void __launch_bounds__(PS_THREADS, 1) k_cg_rows(CgArgs a, int R) {
+    extern __shared__ __align__(16) double sm[];
+    __shared__ double red[PS_THREADS / 32], um_s[2], quot;
+    constexpr int NW = PS_THREADS / 32;
+    const int G = gridDim.x, bx = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int P = (int)a.P, Ns = a.Ns, r0 = bx * R, nr = max(0, min(R, Ns - r0)), items = TWO ? 2 * nr : nr;
+    double *rows = sm, *ps = rows + (size_t)(TWO ? 2 : 1) * R * P, *us = ps + P;   // row nr + i: row i of O2
+    const int S = items > 0 ? max(1, NW / items) : 1;       // warps a row
+    double *up = us + 2 * R;                                // [items][S] partial row dots
+    for (int e = tid; e < nr * P; e += PS_THREADS) {
+        rows[e] = a.O[(size_t)r0 * P + e];
+        if (TWO) rows[(size_t)nr * P + e] = a.O2[(size_t)r0 * P + e];
+    }
+    double p[E], r[E], d[E];
+    double s = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const int k = tid + PS_THREADS * e;
+        p[e] = r[e] = k < P ? a.F[k] : 0.0;
+        d[e] = 0.0;
+        if (k < P) ps[k] = p[e];
+        s = fma(r[e], r[e], s);
+    }
+    const double rs0 = cg_block_sum(s, red);
+    double rs = rs0, pap_last = 0.0;
+    int it = 0, done = 0, conv = 0;
+    // partials of CTA b: P columns, then sum u and sum u2 of its rows
+    double *const part = a.upart + (size_t)bx * (P + 2);
+    for (; it < a.max_iters; it++) {
+        for (int w = warp; w < items * S; w += NW) {
+            const int i = w / S, q = w % S;
+            const double *row = rows + (size_t)i * P;
+            double x0 = 0.0, x1 = 0.0, x2 = 0.0, x3 = 0.0;
+            int k = q * 32 + lane;
+            const int st = 32 * S;
+            for (; k + 3 * st < P; k += 4 * st) {
+                x0 = fma(row[k], ps[k], x0);
+                x1 = fma(row[k + st], ps[k + st], x1);
+                x2 = fma(row[k + 2 * st], ps[k + 2 * st], x2);
+                x3 = fma(row[k + 3 * st], ps[k + 3 * st], x3);
+            }
+            for (; k < P; k += st) x0 = fma(row[k], ps[k], x0);
+            x0 = warp_sum((x0 + x1) + (x2 + x3));
+            if (lane == 0) up[w] = x0;
+        }
+        __syncthreads();
+        if (tid < items) {
+            double v = up[tid * S];
+            for (int q = 1; q < S; q++) v += up[tid * S + q];
+            us[tid] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int k = tid + PS_THREADS * e;
+            if (k < P) {
+                double x = 0.0, y = 0.0;
+                for (int i = 0; i < nr; i++) x = fma(rows[(size_t)i * P + k], us[i], x);
+                for (int i = nr; i < items; i++) y = fma(rows[(size_t)i * P + k], us[i], y);
+                part[k] = TWO ? x + y : x;
+            }
+        }
+        if (tid < (TWO ? 2 : 1)) {
+            double v = 0.0;
+            for (int i = 0; i < nr; i++) v += us[tid * nr + i];
+            part[P + tid] = v;
+        }
+        if (!grid_barrier(a.bar, a.err, G)) return;
+        // columns bx, bx + G, ... of A p, a warp each; the last warp also forms <u>, <u2>
+        if (warp == NW - 1) {
+            double v = 0.0, v2 = 0.0;
+            for (int g = lane; g < G; g += 32) {
+                v += __ldcg(a.upart + (size_t)g * (P + 2) + P);
+                if (TWO) v2 += __ldcg(a.upart + (size_t)g * (P + 2) + P + 1);
+            }
+            v = warp_sum(v);
+            if (TWO) v2 = warp_sum(v2);
+            if (lane == 0) {
+                um_s[0] = v / (double)Ns;
+                um_s[1] = TWO ? v2 / (double)Ns : 0.0;
+            }
+        }
+        for (int k0 = bx + G * warp; k0 - G * warp < P; k0 += G * NW) {      // the same trip count in all warps
+            double v = 0.0;
+            if (k0 < P)
+                for (int g = lane; g < G; g += 32) v += __ldcg(a.upart + (size_t)g * (P + 2) + k0);
+            v = warp_sum(v);
+            __syncthreads();                                                 // um_s
+            if (lane == 0 && k0 < P) {
+                // the mean terms rounded before they are taken off, as upstream does
+                v = __dsub_rn(v / (double)Ns, __dmul_rn(a.gm[k0], um_s[0]));
+                if (TWO) v = a.fac * __dsub_rn(v, __dmul_rn(a.gm2[k0], um_s[1]));
+                a.Ap[k0] = fma(a.eps, ps[k0], v);
+            }
+        }
+        if (!grid_barrier(a.bar, a.err, G)) return;
+        double ap[E];
+        s = 0.0;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int k = tid + PS_THREADS * e;
+            ap[e] = k < P ? __ldcg(a.Ap + k) : 0.0;
+            s = fma(p[e], ap[e], s);
+        }
+        const double pap = cg_block_sum(s, red);
+        if (!(fabs(pap) >= 1e-30)) {                        // Krylov breakdown: stop, unconverged
+            done = 1;
+            pap_last = pap;
+            break;
+        }
+        if (tid == 0) quot = rs / pap;                      // one thread: a division is seven FP64 instructions
+        __syncthreads();
+        const double alpha = quot;
+        s = 0.0;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            if (bx == 0) d[e] = fma(alpha, p[e], d[e]);
+            r[e] = fma(-alpha, ap[e], r[e]);
+            s = fma(r[e], r[e], s);
+        }
+        const double rs_new = cg_block_sum(s, red);
+        if (rs_new <= a.tol * a.tol * rs0) {
+            done = 1;
+            conv = 1;
+            it++;
+            break;
+        }
+        if (tid == 0) quot = rs_new / rs;
+        __syncthreads();
+        const double beta = quot;
+        rs = rs_new;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int k = tid + PS_THREADS * e;
+            p[e] = fma(beta, p[e], r[e]);
+            if (k < P) ps[k] = p[e];
+        }
+        __syncthreads();
+    }
+    if (bx == 0) {
+#pragma unroll
+        for (int e = 0; e < E; e++)
+            if (tid + PS_THREADS * e < P) a.d[tid + PS_THREADS * e] = d[e];
+        if (tid == 0) {
+            a.scal[S_RS] = rs;
+            a.scal[S_RS0] = rs0;
+            a.scal[S_PAP] = pap_last;
+            a.status[I_DONE] = done;
+            a.status[I_CONV] = conv;
+            a.status[I_ITERS] = it;
+        }
+    }
+}
+
+// Shared memory of k_cg_rows at R rows a CTA.
+static size_t cg_rows_smem(int R, long P, bool two) {
+    return sizeof(double) * ((size_t)(two ? 2 : 1) * R * P + P + 2 * R + std::max(2 * R, PS_THREADS / 32));
+}
+
 bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double *gm, double eps, double tol,
                  int max_iters, double *d, double *scal, int *status, const double *O2, const double *gm2,
                  double fac) {
@@ -2654,8 +2839,14 @@ bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double 
     static DevBuf<double> r, p, Ap, u, upart, u2, upart2;
     static DevBuf<unsigned> bar;
     static DevBuf<int> err;
+    // rows in shared memory where they fit: at least four a CTA (fewer would only add CTAs to the
+    // barriers: 256 x 288 takes the same time on 64 CTAs as on 152)
+    const int R = std::max(4, (Ns + c.sm_count - 1) / c.sm_count), Gr = (Ns + R - 1) / R;
+    const size_t rsm = cg_rows_smem(R, P, O2 != nullptr);
+    const bool in_smem = P <= CG_MAX_P && rsm <= 224 * 1024;
     if (!r.ensure(P) || !p.ensure(P) || !Ap.ensure(P) || !u.ensure(Ns) ||
-        !upart.ensure((size_t)((Ns + RCH - 1) / RCH) * P) || !bar.ensure(2) || !err.ensure(1) ||
+        !upart.ensure(std::max((size_t)((Ns + RCH - 1) / RCH) * P, in_smem ? (size_t)Gr * (P + 2) : 0)) ||
+        !bar.ensure(2) || !err.ensure(1) ||
         (O2 && (!u2.ensure(Ns) || !upart2.ensure((size_t)((Ns + RCH - 1) / RCH) * P))))
         return false;
     if (!NQS_CUDA(cudaMemsetAsync(bar.p, 0, 2 * sizeof(unsigned), st)) ||
@@ -2663,23 +2854,28 @@ bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double 
         return false;
     CgArgs a{O,   Ns,  P,   F,    gm,      O2,   gm2,      fac,  eps,   tol,   max_iters, d,
              r.p, p.p, Ap.p, u.p, upart.p, u2.p, upart2.p, scal, status, bar.p, err.p};
+    void (*krows)(CgArgs, int) = nullptr;
+    if (in_smem) {
+        const int E = (int)((P + PS_THREADS - 1) / PS_THREADS);
+        if (O2) krows = E <= 1 ? k_cg_rows<1, true> : E <= 2 ? k_cg_rows<2, true> : E <= 4 ? k_cg_rows<4, true> : k_cg_rows<8, true>;
+        else krows = E <= 1 ? k_cg_rows<1, false> : E <= 2 ? k_cg_rows<2, false> : E <= 4 ? k_cg_rows<4, false> : k_cg_rows<8, false>;
+        if (!NQS_CUDA(cudaFuncSetAttribute(krows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm))) return false;
+    }
     int per_sm = 0;
     if (!NQS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_sr, PS_THREADS, 0))) return false;
     if (per_sm < 1) {
         set_error("CG kernel does not fit on an SM");
         return false;
     }
-    // one CTA per 256 KB of Jacobian (at least 8, at most one per SM): a small system
-    // (the 1-D TFIM chain: 1024 x 288, 2.4 MB) then synchronises 10 CTAs instead of 152 at
-    // its five grid barriers per iteration; the dot products run in every CTA in a fixed
-    // order and the column sums are reduced over fixed row chunks, so the result does not
-    // depend on the grid size
+    // k_cg_sr: one CTA per 256 KB of Jacobian (at least 8, at most one per SM); the dot
+    // products run in every CTA in a fixed order and the column sums are reduced over fixed row
+    // chunks, so the result does not depend on the grid size
     const double jac_bytes = 8.0 * (double)Ns * (double)P * (O2 ? 2.0 : 1.0);
     const int grid = std::max(8, std::min(c.sm_count, (int)std::ceil(jac_bytes / (256.0 * 1024.0))));
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)grid);
+    lc.gridDim = dim3((unsigned)(in_smem ? Gr : grid));
     lc.blockDim = dim3(PS_THREADS);
-    lc.dynamicSmemBytes = 0;
+    lc.dynamicSmemBytes = in_smem ? rsm : 0;
     lc.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -2688,7 +2884,7 @@ bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double 
     lc.numAttrs = 1;
     {
         NQS_LAUNCH("cg_sr");
-        if (!NQS_CUDA(cudaLaunchKernelEx(&lc, k_cg_sr, a))) return false;
+        if (!NQS_CUDA(in_smem ? cudaLaunchKernelEx(&lc, krows, a, R) : cudaLaunchKernelEx(&lc, k_cg_sr, a))) return false;
     }
     int herr = 0;
     if (!NQS_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
