@@ -334,7 +334,8 @@ typedef struct {
      * other CTAs and [2] CTA 0's own chain of diagonal-block steps, otherwise [1] panels
      * and [2] trailing updates (each with the next diagonal block's update and factor by
      * CTA 0 beside the trailing tiles); [3] the last block row of L^{-1} (or the whole
-     * inverse); [4] preconditioner applications, [5] right-hand side and operator
+     * inverse); [4] preconditioner applications (above order 4608
+     * with the inverses of its 1024-wide blocks), [5] right-hand side and operator
      * products, [6] total (the CG vector updates and dot products are the rest of it);
      * [7] the time CTA 0 spent on its diagonal-block steps (summed over the blocks) */
     double phase_us[8];

@@ -1134,6 +1134,12 @@ __device__ bool trailing_tile_tc(TcState &ts, const float *ah, const float *al, 
 // Order from which the preconditioner is applied by blocked substitution
 // instead of through an explicit L^{-1}.
 constexpr int BLOCKED_SOLVE_MIN = 4608;
+// Superblock of that substitution: the inverses of the SB-wide diagonal blocks of L are formed after
+// the factor (6 GFLOP of SIMT tiles at n = 8192), so a direction takes two grid barriers per 1024
+// columns and every row of a phase is read by one warp, where the BD-wide blocks took a barrier per
+// 128 columns and every CTA read each diagonal block.  Measured: n = 8192, seven applications: 1.60 ms
+// and 0.25 ms for the inverses, against 10.05 ms; n = 15014, six: 3.47 + 0.41 against 17.4 ms.
+constexpr int SB = 1024;
 
 // Relative residual |r| / |rhs| at which the CG refinement stops.
 constexpr double CG_RTOL = 1e-10;
@@ -1260,9 +1266,8 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
         if (tid == 0 && a.tm) atomicAdd(a.tm + 7, gtimer() - t_own);
     };
     // Large systems skip the explicit L^{-1} (n^3 / 3 flops) and apply the
-    // preconditioner by blocked substitution (one grid barrier per diagonal
-    // block and direction); below BLOCKED_SOLVE_MIN the inverse is cheaper than
-    // those barriers over the CG iterations.
+    // preconditioner by substitution over SB-wide blocks (two grid barriers per block and
+    // direction); below BLOCKED_SOLVE_MIN the inverse is built beside the factor.
     const bool blocked = n >= BLOCKED_SOLVE_MIN;
     // X = L^{-1} is built beside the factor (forward substitution of L X = I, right-looking
     // by block columns): R = I - sum_{p < kb} L_{:,p} X_{p,:} accumulates in the lower
@@ -1647,6 +1652,50 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
         if (!grid_barrier(a.bar, a.err, G)) return;
     }
     NQS_PHASE(3);
+    // ---------------- inverses of the SB-wide diagonal superblocks of L (large systems): from the
+    // BD-wide ones by doubling, X21 = -X22 (L21 X11), every pair of every superblock at once.  L21 is
+    // U = L^T in the upper triangle of T; W = L21 X11 goes to T's lower triangle, dead since the factor.
+    if (blocked) {
+        for (int m = BD; m < SB && m < n; m *= 2) {
+            const int mt = m / GT, per = mt * mt, np = (n - m + 2 * m - 1) / (2 * m);
+            for (int t = bx; t < np * per; t += G) {
+                const int q0 = t / per * 2 * m, i0 = q0 + m + t % per / mt * GT, j0 = q0 + t % mt * GT;
+                if (i0 >= n) continue;
+                float acc[4][4] = {};
+                gemm64<true, true>(acc, a.T, n, i0, n, a.Li, ldl, j0, q0 + m, j0, q0 + m, TS);
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int v = 0; v < 4; v++) {
+                        const int i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
+                        if (i < n) a.T[(size_t)i * n + j] = acc[u][v];
+                    }
+            }
+            if (!grid_barrier(a.bar, a.err, G)) return;
+            for (int t = bx; t < np * per; t += G) {
+                const int q0 = t / per * 2 * m, i0 = q0 + m + t % per / mt * GT, j0 = q0 + t % mt * GT;
+                if (i0 >= n) continue;
+                float acc[4][4] = {};
+                gemm64<false, true>(acc, a.Li, ldl, i0, n, a.T, n, j0, q0 + m, q0 + m, min(n, i0 + GT), TS);
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int v = 0; v < 4; v++) {
+                        const int i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
+                        if (i < n) a.Li[(size_t)i * ldl + j] = -acc[u][v];
+                        ST[ty + 16 * u][tx + 16 * v] = -acc[u][v];
+                    }
+                __syncthreads();
+                for (int e = tid; e < GT * GT; e += PS_THREADS) {
+                    const int jj = e / GT, ii = e % GT;
+                    if (i0 + ii < n) a.LiT[(size_t)(j0 + jj) * ldl + i0 + ii] = ST[ii][jj];
+                }
+                __syncthreads();
+            }
+            if (!grid_barrier(a.bar, a.err, G)) return;
+        }
+    }
+    NQS_PHASE(4);
 
     const int Ns = a.Ns;
     const long P = a.P;
@@ -1857,89 +1906,79 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
     // M^{-1} v with rf = float(v): zf = L^{-1} rf, out = L^{-T} zf (row i of
     // L^{-1} reads the 4-aligned groups up to i; the entries right of the
     // diagonal inside a group are the zeros of the diagonal block).
-    __shared__ float vk[BD], yk[BD];
+    __shared__ float vred[PS_THREADS / 32][33];
     auto precond = [&](double *out) -> bool {
         if (blocked) {
             const int warp = tid >> 5;
-            constexpr int RL = BD / 32;
-            // yk[t] = sum_c X[t][c] vk[c] over the diagonal block (rows of X at
-            // xb + t * ldl; the zeros of the triangle are read too), a warp
-            // taking 4 rows at a time with all their loads issued first
-            auto diag_gemv = [&](const float *xb, int bs) {
-                for (int c = bs + tid; c < BD; c += PS_THREADS) vk[c] = 0.f;
-                __syncthreads();
-                for (int t0 = 4 * warp; t0 < bs; t0 += 4 * (PS_THREADS / 32)) {
-                    float xv[4][RL];
-#pragma unroll
-                    for (int h = 0; h < 4; h++)
-#pragma unroll
-                        for (int q = 0; q < RL; q++) {
-                            const int t = t0 + h, c = lane + 32 * q;
-                            xv[h][q] = (t < bs && c < bs) ? __ldcg(xb + (size_t)t * ldl + c) : 0.f;
-                        }
-#pragma unroll
-                    for (int h = 0; h < 4; h++) {
-                        float sacc = 0.f;
-#pragma unroll
-                        for (int q = 0; q < RL; q++) sacc = fmaf(xv[h][q], vk[lane + 32 * q], sacc);
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-                        if (lane == 0 && t0 + h < bs) yk[t0 + h] = sacc;
-                    }
+            // forward, L y = rf (rf is the working vector): y_s = X_s w_s by rows, then
+            // w_i -= sum_c L[i][s0 + c] y_c = sum_c U[s0 + c][i] y_c below the superblock, 32 rows i a
+            // CTA with the columns split over its warps (coalesced over i, 32 loads in flight)
+            for (int s0 = 0; s0 < n; s0 += SB) {
+                const int s1 = min(n, s0 + SB);
+                for (int i = s0 + gwarp; i < s1; i += gwarps) {
+                    const float t = dot4_range(a.Li + (size_t)i * ldl, a.rf, s0 >> 2, (i >> 2) + 1, lane);
+                    if (lane == 0) a.zf[i] = t;
                 }
-                for (int t = bs + tid; t < BD; t += PS_THREADS) yk[t] = 0.f;   // read (times 0) past a partial block
+                if (!grid_barrier(a.bar, a.err, G)) return false;
+                if (s1 == n) break;
+                float *ys = psm;                                // y_s; the superblock is whole (s1 < n)
+                if (s1 + 32 * bx < n)
+                    for (int c = tid; c < SB; c += PS_THREADS) ys[c] = __ldcg(a.zf + s0 + c);
                 __syncthreads();
-            };
-            // forward, L y = rf (rf is the working vector): y_k = X_kk w_k, then
-            // w_i -= sum_c L[i][k0 + c] y_k[c] = sum_c U[k0 + c][i] y_k[c] below the block
-            for (int kb = 0; kb < nb; kb++) {
-                const int k0 = kb * BD, bs = min(BD, n - k0), k1 = k0 + bs;
-                for (int c = tid; c < bs; c += PS_THREADS) vk[c] = __ldcg(a.rf + k0 + c);
-                diag_gemv(a.Li + (size_t)k0 * ldl + k0, bs);      // X_kk (lower triangle)
-                if (bx == 0)
-                    for (int c = tid; c < bs; c += PS_THREADS) a.zf[k0 + c] = yk[c];
-                for (int i = k1 + gtid; i < n; i += gthreads) {
-                    // 32 loads in flight per round (coalesced over i)
-                    const float *u = a.T + (size_t)k0 * n + i;
-                    float sacc = 0.f;
-                    for (int c0 = 0; c0 < bs; c0 += 32) {
-                        float uv[32];
+                for (int i0 = s1 + 32 * bx; i0 < n; i0 += 32 * G) {
+                    const int i = i0 + lane;
+                    constexpr int SEG = SB / (PS_THREADS / 32);
+                    const int c0 = warp * SEG;
+                    float acc = 0.f;
+                    if (i < n) {
+                        const float *u = a.T + (size_t)(s0 + c0) * n + i;
+                        for (int c = 0; c < SEG; c += 32) {
+                            float uv[32];
 #pragma unroll
-                        for (int q = 0; q < 32; q++) uv[q] = c0 + q < bs ? __ldcg(u + (size_t)(c0 + q) * n) : 0.f;
+                            for (int q = 0; q < 32; q++) uv[q] = __ldcg(u + (size_t)(c + q) * n);
 #pragma unroll
-                        for (int q = 0; q < 32; q++) sacc = fmaf(uv[q], yk[min(c0 + q, BD - 1)], sacc);
+                            for (int q = 0; q < 32; q++) acc = fmaf(uv[q], ys[c0 + c + q], acc);
+                        }
                     }
-                    a.rf[i] = __ldcg(a.rf + i) - sacc;
+                    vred[warp][lane] = acc;
+                    __syncthreads();
+                    if (warp == 0 && i < n) {
+                        float t = 0.f;
+#pragma unroll
+                        for (int w = 0; w < PS_THREADS / 32; w++) t += vred[w][lane];
+                        a.rf[i] = __ldcg(a.rf + i) - t;
+                    }
+                    __syncthreads();
                 }
                 if (!grid_barrier(a.bar, a.err, G)) return false;
             }
-            // backward, L^T z = y (zf is the working vector): z_k = X_kk^T v_k, then
-            // v_i -= sum_r L[k0 + r][i] z_k[r] = sum_r U[i][k0 + r] z_k[r] above the block
-            for (int kb = nb - 1; kb >= 0; kb--) {
-                const int k0 = kb * BD, bs = min(BD, n - k0);
-                for (int c = tid; c < bs; c += PS_THREADS) vk[c] = __ldcg(a.zf + k0 + c);
-                diag_gemv(a.LiT + (size_t)k0 * ldl + k0, bs);     // X_kk^T (upper triangle)
-                if (bx == 0)
-                    for (int c = tid; c < bs; c += PS_THREADS) out[k0 + c] = (double)yk[c];
-                // a warp takes 4 rows at a time, all BD / 32 loads per row issued first
-                for (int i0 = 4 * gwarp; i0 < k0; i0 += 4 * gwarps) {
-                    float uv[4][RL];
-#pragma unroll
-                    for (int h = 0; h < 4; h++)
-#pragma unroll
-                        for (int q = 0; q < RL; q++) {
-                            const int r = lane + 32 * q;
-                            uv[h][q] = (i0 + h < k0 && r < bs) ? __ldcg(a.T + (size_t)(i0 + h) * n + k0 + r) : 0.f;
-                        }
-#pragma unroll
-                    for (int h = 0; h < 4; h++) {
-                        float sacc = 0.f;
-#pragma unroll
-                        for (int q = 0; q < RL; q++) sacc = fmaf(uv[h][q], yk[lane + 32 * q], sacc);
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-                        if (lane == 0 && i0 + h < k0) a.zf[i0 + h] = __ldcg(a.zf + i0 + h) - sacc;
+            // backward, L^T z = y (zf is the working vector): z_s = X_s^T v_s by rows of LiT, then
+            // v_i -= sum_r L[s0 + r][i] z_r = sum_r U[i][s0 + r] z_r above the superblock, a warp a row
+            for (int s0 = (n - 1) / SB * SB; s0 >= 0; s0 -= SB) {
+                const int s1 = min(n, s0 + SB);
+                for (int j = s0 + gwarp; j < s1; j += gwarps) {
+                    const float t = dot4_range(a.LiT + (size_t)j * ldl, a.zf, j >> 2, (s1 + 3) >> 2, lane);
+                    if (lane == 0) {
+                        out[j] = (double)t;
+                        a.rf[j] = t;
                     }
+                }
+                if (!grid_barrier(a.bar, a.err, G)) return false;
+                if (s0 == 0) break;
+                float *zs = psm;                                // z_s
+                for (int r = tid; r < SB; r += PS_THREADS) zs[r] = s0 + r < s1 ? __ldcg(a.rf + s0 + r) : 0.f;
+                __syncthreads();
+                for (int i = gwarp; i < s0; i += gwarps) {
+                    const float *u = a.T + (size_t)i * n;
+                    float acc = 0.f;
+                    float uv[SB / 32];
+#pragma unroll
+                    for (int q = 0; q < SB / 32; q++) uv[q] = s0 + lane + 32 * q < s1 ? __ldcg(u + s0 + lane + 32 * q) : 0.f;
+#pragma unroll
+                    for (int q = 0; q < SB / 32; q++) acc = fmaf(uv[q], zs[lane + 32 * q], acc);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                    if (lane == 0) a.zf[i] = __ldcg(a.zf + i) - acc;
                 }
                 if (!grid_barrier(a.bar, a.err, G)) return false;
             }
