@@ -61,8 +61,8 @@ struct GramTcArgs {
     int kt_per_seg;       // K tiles per CTA: kt_total, or a third of it in a split launch
     int nseg;             // products: 1 = hi hi^T, 3 = hi hi^T + hi lo^T + lo hi^T
     float scale, shift;
-    float *C;             // [n][n] lower triangle written
-    int n;
+    float *C;             // [n][ldc] lower triangle written (a split launch's partials: [n][n])
+    int n, ldc;
     int *err;
     int split;            // 1: blockIdx.y = K segment, raw partial sums into C + segment * n * n
 };
@@ -181,7 +181,7 @@ k_gram_tf32_tc(const __grid_constant__ CUtensorMap map_hi, const __grid_constant
                     if (col <= row && col < g.n) dst[col] = v[j];
                 }
             } else if (row < g.n) {
-                float *dst = g.C + (size_t)row * g.n;
+                float *dst = g.C + (size_t)row * g.ldc;
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
                     int col = col0 + j;
@@ -200,13 +200,13 @@ k_gram_tf32_tc(const __grid_constant__ CUtensorMap map_hi, const __grid_constant
 // T = scale ((P0 + P1) + P2) + shift I on the lower triangle, from the three
 // K-segment partial Grams of a split launch (rows dealt to the blocks, columns c <= r to
 // the threads).
-__global__ void k_gram_sum(const float *__restrict__ Pp, int n, float scale, float shift, float *T) {
+__global__ void k_gram_sum(const float *__restrict__ Pp, int n, int ldt, float scale, float shift, float *T) {
     const size_t nn = (size_t)n * n;
     for (int r = blockIdx.x; r < n; r += gridDim.x) {
         const size_t e0 = (size_t)r * n;
         for (int c = threadIdx.x; c <= r; c += blockDim.x) {
             const size_t e = e0 + c;
-            T[e] = ((Pp[e] + Pp[nn + e]) + Pp[2 * nn + e]) * scale + (r == c ? shift : 0.f);
+            T[(size_t)r * ldt + c] = ((Pp[e] + Pp[nn + e]) + Pp[2 * nn + e]) * scale + (r == c ? shift : 0.f);
         }
     }
 }
@@ -323,7 +323,10 @@ static_assert(BD_SMALL % 64 == 0 && BD_LARGE <= BT, "diagonal blocks are multipl
 constexpr int PS_THREADS = 256;
 constexpr int DF_G = 9;           // four-column groups per lane in flight in a row dot of the operator
 constexpr int DF_SEGS = 4;        // row segments of a chunk at most in the operator's column sums
-constexpr int PS_SMEM = 2 * BT * (BT + 1) * 4;       // two 128 x 129 float tiles
+// two 128 x 129 float tiles; the rank-update tiles' two operand stages (64 KB each) and tile of T,
+// 1024-byte aligned (with the static shared memory 230752 of the 232448 bytes a block may have)
+constexpr int PS_SMEM = 1024 + 2 * 4 * 128 * 32 * 4 + 128 * 132 * 4;
+static_assert(PS_SMEM >= 2 * BT * (BT + 1) * 4, "two tiles of the diagonal block");
 constexpr int GT = 64, GKC = 32;                     // GEMM tile and K chunk
 constexpr int RCH = 64;                              // rows per partial column sum
 
@@ -987,147 +990,152 @@ __device__ __forceinline__ void stage_sw128(uint32_t sbase, const float *X, int 
 }
 
 struct TcState {
-    uint8_t *sm;          // 2 stages of TT_STAGE_BYTES, 1024-byte aligned (also the epilogue tile)
+    uint8_t *sm;          // 2 stages of TT_STAGE_BYTES, 1024-byte aligned, and a 128 x 132 tile of T
     uint64_t *mbar;       // [2] MMA completion per stage
     uint32_t cnt[2];      // commits issued per stage (mbarrier phase tracking)
     uint32_t tmem;        // 128 TMEM columns (128 x 128 FP32 accumulator)
     int *err;
 };
 
-// One 128 x 128 tile of a rank-BD update, C = A_i B_j^T over K = BD with the operands
+// 128 x 128 tiles of a rank-BD update, C = A_i B_j^T over K = BD with the operands
 // rows R0 .. R0 + 127 of (ah, al) and C0 .. C0 + 127 of (bh, bl) ([row][BD] TF32 hi / lo).
-// Trailing mode (lim == 0): T[i][j] -= C for j <= i < n (row pitch n), except the entries
-// with i, j < skip (the next diagonal block, updated by its owner).  Inverse mode
-// (lim > 0): T[i][j] -= C for i < n, j < lim (row pitch ldt), where the columns j >= skip
-// take their first update (T = -C, nothing read).  Returns false when a bounded wait gave
-// up (err raised).
-template <int BD>
-__device__ bool trailing_tile_tc(TcState &ts, const float *ah, const float *al, const float *bh, const float *bl,
-                                 float *T, int n, int ldt, int R0, int C0, int skip, int lim) {
-    constexpr int NQ = BD / 32;
+// Trailing mode (lim == 0): T[i][j] -= C for j <= i < n, except the entries with i, j < skip (the
+// next diagonal block, updated by its owner).  Inverse mode (lim > 0): T[i][j] -= C for i < n,
+// j < lim, where the columns j >= skip take their first update (T = -C, nothing read).  T, lim and
+// skip are in multiples of 4 columns of 16-byte aligned rows, so no float4 group straddles them
+// but at the diagonal.
+struct TileJob {
+    const float *ah, *al, *bh, *bl;
+    float *T;
+    int R0, C0, skip, lim;
+};
+
+// Tiles t0, t0 + dt, ... < nall of the step, job(t) describing each and done(t) called after its
+// stores.  The tiles follow each other without a gap in the operand stream: while tile t's values of T
+// (fetched beside its MMAs into a tile of their own in shared memory) are updated and stored, the
+// first two K chunks of the next tile are in flight.  Bound by the bytes an SM takes from L2 (320 KB a
+// tile at BD = 128, about 60 bytes a clock) rather than by the MMAs.  Measured, order 15014:
+// MEAS_RU a tile; with every tile on its own (operands, then T, then stores) 13 us.  Returns false
+// when a bounded wait gave up (err raised).
+template <int BD, typename Job, typename Done>
+__device__ __forceinline__ bool rank_update_tiles(TcState &ts, int n, int ldt, int t0, int dt, int nall, Job job,
+                                                  Done done) {
+    constexpr int NQ = BD / 32, EP = TT + 4;                // EP: 16-byte rows, conflict-free 128-bit accesses
+    static_assert(NQ == 2 || NQ == 4, "chunk q of every tile goes to buffer q % 2");
+    if (t0 >= nall) return true;
     const int tid = threadIdx.x;
     const uint32_t s0 = smem_u32(ts.sm);
-    auto stage = [&](int q, int b) {
-        const uint32_t sb = s0 + b * TT_STAGE_BYTES;
-        stage_sw128<BD>(sb, ah, R0, q);
-        stage_sw128<BD>(sb + TT_CHUNK_BYTES, al, R0, q);
-        stage_sw128<BD>(sb + 2 * TT_CHUNK_BYTES, bh, C0, q);
-        stage_sw128<BD>(sb + 3 * TT_CHUNK_BYTES, bl, C0, q);
+    float *tb = (float *)(ts.sm + 2 * TT_STAGE_BYTES);      // the tile of T
+    auto stage = [&](const TileJob &w, int q) {
+        const uint32_t sb = s0 + (q & 1) * TT_STAGE_BYTES;
+        stage_sw128<BD>(sb, w.ah, w.R0, q);
+        stage_sw128<BD>(sb + TT_CHUNK_BYTES, w.al, w.R0, q);
+        stage_sw128<BD>(sb + 2 * TT_CHUNK_BYTES, w.bh, w.C0, q);
+        stage_sw128<BD>(sb + 3 * TT_CHUNK_BYTES, w.bl, w.C0, q);
         cp_async_commit();
     };
+    auto mma_done = [&](int b) { return mbar_wait(&ts.mbar[b], (ts.cnt[b] - 1) & 1, ts.err); };
     // M = N = 128, FP32 accumulate, TF32 operands, both K-major
     const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TT >> 3) << 17) | ((uint32_t)(TT >> 4) << 24);
-    stage(0, 0);
-    for (int q = 0; q < NQ; q++) {
-        const int b = q & 1;
-        cp_async_wait_all();
-        fence_proxy_async();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t sb = s0 + b * TT_STAGE_BYTES;
+    TileJob w = job(t0);
+    stage(w, 0);
+    stage(w, 1);
+    for (int t = t0; t < nall; t += dt) {
 #pragma unroll
-            for (int pass = 0; pass < 3; pass++) {
-                const uint32_t sa = sb + (pass == 2 ? TT_CHUNK_BYTES : 0);                       // A hi, hi, lo
-                const uint32_t sbb = sb + 2 * TT_CHUNK_BYTES + (pass == 1 ? TT_CHUNK_BYTES : 0);  // B hi, lo, hi
+        for (int q = 0; q < 16; q++) {
+            const int e4 = tid + q * PS_THREADS, r = e4 >> 5, c = 4 * (e4 & 31), i = w.R0 + r, j = w.C0 + c;
+            if (i < n && (w.lim > 0 ? j < w.lim && j < w.skip : j <= i))
+                cp_async16(smem_u32(tb + r * EP + c), &w.T[(size_t)i * ldt + j]);
+            else if (w.lim > 0)
+                *(float4 *)&tb[r * EP + c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        cp_async_commit();
+        // groups in flight: chunks 0, 1, the tile of T, then chunks 2, 3 as their buffers come free
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    umma_tf32(ts.tmem, sw128_desc(sa + k * 32), sw128_desc(sbb + k * 32), idesc,
-                              (q | pass | k) ? 1u : 0u);
+        for (int q = 0; q < NQ; q++) {
+            const int b = q & 1;
+            if (q == 0) cp_async_wait<2>();
+            else if (q == 1) cp_async_wait<1>();
+            else cp_async_wait<0>();
+            fence_proxy_async();
+            __syncthreads();
+            if (tid == 0) {
+                tc_fence_after();
+                const uint32_t sb = s0 + b * TT_STAGE_BYTES;
+#pragma unroll
+                for (int pass = 0; pass < 3; pass++) {
+                    const uint32_t sa = sb + (pass == 2 ? TT_CHUNK_BYTES : 0);                       // A hi, hi, lo
+                    const uint32_t sbb = sb + 2 * TT_CHUNK_BYTES + (pass == 1 ? TT_CHUNK_BYTES : 0);  // B hi, lo, hi
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        umma_tf32(ts.tmem, sw128_desc(sa + k * 32), sw128_desc(sbb + k * 32), idesc,
+                                  (q | pass | k) ? 1u : 0u);
+                }
+                umma_commit(&ts.mbar[b]);
             }
-            umma_commit(&ts.mbar[b]);
-        }
-        ts.cnt[b]++;
-        if (q + 1 < NQ) {
-            const int nb = (q + 1) & 1;
-            // the stage being refilled was read by the MMAs of chunk q - 1
-            if (q >= 1 && !__syncthreads_and(mbar_wait(&ts.mbar[nb], (ts.cnt[nb] - 1) & 1, ts.err))) return false;
-            stage(q + 1, nb);
-        }
-    }
-    const int lb = (NQ - 1) & 1;
-    bool done = mbar_wait(&ts.mbar[lb], (ts.cnt[lb] - 1) & 1, ts.err);
-    if (NQ > 1) done = done && mbar_wait(&ts.mbar[lb ^ 1], (ts.cnt[lb ^ 1] - 1) & 1, ts.err);
-    if (!__syncthreads_and(done)) return false;             // uniform over the CTA
-    tc_fence_after();
-    // epilogue: warp w reads TMEM lanes 32 (w % 4) .., columns 64 (w / 4) .. + 63
-    // into a shared tile of pitch EP (16-byte rows: conflict-free 128-bit
-    // accesses), then the tile is subtracted from T with coalesced accesses
-    constexpr int EP = TT + 4;
-    float *ep = (float *)ts.sm;
-    {
-        const int warp = tid >> 5, lane = tid & 31, row = 32 * (warp & 3) + lane;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int col = 64 * (warp >> 2) + 32 * h;
-            float v[32];
-            tmem_ld32(ts.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col, v);
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *(float4 *)&ep[row * EP + col + j] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (lim > 0) {
-        // inverse mode: ldt, lim and skip are multiples of 4, so no float4 group straddles them
-        float4 v[16];
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int e4 = tid + q * PS_THREADS, i = R0 + (e4 >> 5), j = C0 + 4 * (e4 & 31);
-            v[q] = (i < n && j < lim && j < skip) ? __ldcg((const float4 *)&T[(size_t)i * ldt + j])
-                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int e4 = tid + q * PS_THREADS, r = e4 >> 5, c = 4 * (e4 & 31), i = R0 + r, j = C0 + c;
-            if (i < n && j < lim) {
-                const float4 d = *(const float4 *)&ep[r * EP + c];
-                *(float4 *)&T[(size_t)i * ldt + j] = make_float4(v[q].x - d.x, v[q].y - d.y, v[q].z - d.z, v[q].w - d.w);
+            ts.cnt[b]++;
+            if (q >= 1 && q + 1 < NQ) {                     // the MMAs of chunk q - 1 have read its buffer
+                if (!__syncthreads_and(mma_done(b ^ 1))) return false;
+                stage(w, q + 1);
             }
         }
-    } else if ((n & 3) == 0) {
-        // 16 float4 per thread, all loads before the stores
-        float4 v[16];
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int e4 = tid + q * PS_THREADS, i = R0 + (e4 >> 5), j = C0 + 4 * (e4 & 31);
-            v[q] = (i < n && j <= i) ? __ldcg((const float4 *)&T[(size_t)i * n + j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!__syncthreads_and(mma_done(1) && mma_done(0))) return false;
+        tc_fence_after();
+        const bool more = t + dt < nall;
+        TileJob nx = w;
+        if (more) {
+            nx = job(t + dt);
+            stage(nx, 0);
+            stage(nx, 1);
         }
+        if (NQ == 2) {                                      // the tile of T (waited for with chunk 2 when NQ = 4)
+            if (more) cp_async_wait<2>();
+            else cp_async_wait<0>();
+            __syncthreads();
+        }
+        // warp w takes TMEM lanes 32 (w % 4) .., columns 64 (w / 4) .. + 63
+        {
+            const int warp = tid >> 5, lane = tid & 31, row = 32 * (warp & 3) + lane;
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int e4 = tid + q * PS_THREADS, r = e4 >> 5, c = 4 * (e4 & 31), i = R0 + r, j = C0 + c;
-            if (i < n && j <= i && !(i < skip && j < skip)) {   // skip is a multiple of 4 here
-                const float4 d = *(const float4 *)&ep[r * EP + c];
-                float4 o = make_float4(v[q].x - d.x, v[q].y - d.y, v[q].z - d.z, v[q].w - d.w);
-                if (j + 3 <= i) {
-                    *(float4 *)&T[(size_t)i * n + j] = o;
-                } else {                                    // the diagonal crosses this group
-                    float *t = &T[(size_t)i * n + j];
-                    t[0] = o.x;
-                    if (j + 1 <= i) t[1] = o.y;
-                    if (j + 2 <= i) t[2] = o.z;
+            for (int h = 0; h < 2; h++) {
+                const int col = 64 * (warp >> 2) + 32 * h;
+                float v[32];
+                tmem_ld32(ts.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col, v);
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    float4 *p = (float4 *)&tb[row * EP + col + j];
+                    float4 o = *p;
+                    o.x -= v[j];
+                    o.y -= v[j + 1];
+                    o.z -= v[j + 2];
+                    o.w -= v[j + 3];
+                    *p = o;
                 }
             }
         }
-    } else {
-        // 32 independent loads in flight per thread before the stores (a load after
-        // a store to the same array is not hoisted)
-        for (int e0 = tid; e0 < TT * TT; e0 += 32 * PS_THREADS) {
-            float v[32];
+        tc_fence_before();
+        __syncthreads();
 #pragma unroll
-            for (int q = 0; q < 32; q++) {
-                const int e = e0 + q * PS_THREADS, i = R0 + e / TT, j = C0 + e % TT;
-                v[q] = (i < n && j <= i) ? __ldcg(&T[(size_t)i * n + j]) : 0.f;
-            }
-#pragma unroll
-            for (int q = 0; q < 32; q++) {
-                const int e = e0 + q * PS_THREADS, i = R0 + e / TT, j = C0 + e % TT;
-                if (i < n && j <= i && !(i < skip && j < skip)) T[(size_t)i * n + j] = v[q] - ep[(e / TT) * EP + e % TT];
+        for (int q = 0; q < 16; q++) {
+            const int e4 = tid + q * PS_THREADS, r = e4 >> 5, c = 4 * (e4 & 31), i = w.R0 + r, j = w.C0 + c;
+            const float4 o = *(const float4 *)&tb[r * EP + c];
+            float *d = &w.T[(size_t)i * ldt + j];
+            if (w.lim > 0) {
+                if (i < n && j < w.lim) *(float4 *)d = o;
+            } else if (i < n && j <= i && !(i < w.skip && j < w.skip)) {
+                if (j + 3 <= i) {
+                    *(float4 *)d = o;
+                } else {                                    // the diagonal crosses this group
+                    d[0] = o.x;
+                    if (j + 1 <= i) d[1] = o.y;
+                    if (j + 2 <= i) d[2] = o.z;
+                }
             }
         }
+        __syncthreads();                                    // tb is refilled for the next tile
+        done(t);
+        w = nx;
     }
-    __syncthreads();
     return true;
 }
 
@@ -1145,7 +1153,7 @@ constexpr int SB = 1024;
 constexpr double CG_RTOL = 1e-10;
 
 struct FrArgs {
-    float *T;           // [n][n] Gram + shift (lower) on entry; U = L^T in the upper triangle after
+    float *T;           // [n][ldl] Gram + shift (lower) on entry; U = L^T in the upper triangle after
     float *Li, *LiT;    // [n][ldl] L^{-1} (lower; R while it is built) and its transpose; pad columns are zero
     int n;              // order of the system
     int ldl;            // row pitch of Li / LiT (n rounded up to 32)
@@ -1215,8 +1223,8 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
         if (BD == 64) {
             float acc[4][4] = {};
             if (pk0 >= 0) {
-                const float *U = a.T + (size_t)pk0 * n;
-                gemm64<true, true>(acc, U, n, k0, k0 + bs, U, n, k0, k0 + bs, 0, pbs, TS);
+                const float *U = a.T + (size_t)pk0 * ldl;
+                gemm64<true, true>(acc, U, ldl, k0, k0 + bs, U, ldl, k0, k0 + bs, 0, pbs, TS);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++)
@@ -1224,7 +1232,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 for (int v = 0; v < 4; v++) {
                     const int rr = ty + 16 * u, cc = tx + 16 * v;
                     const bool in = rr < bs && cc <= rr;
-                    S0[rr][cc] = in ? __ldcg(&a.T[(size_t)(k0 + rr) * n + k0 + cc]) - acc[u][v]
+                    S0[rr][cc] = in ? __ldcg(&a.T[(size_t)(k0 + rr) * ldl + k0 + cc]) - acc[u][v]
                                     : (rr == cc ? 1.f : 0.f);
                 }
             __syncthreads();
@@ -1236,7 +1244,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 for (int q = 0; q < 8; q++) {
                     const int e = e0 + tid + q * PS_THREADS, rr = e / BD, cc = e % BD;
                     const bool in = e < BD * BD && rr < bs && cc <= rr;
-                    v[q] = in ? __ldcg(&a.T[(size_t)(k0 + rr) * n + k0 + cc]) : (rr == cc ? 1.f : 0.f);
+                    v[q] = in ? __ldcg(&a.T[(size_t)(k0 + rr) * ldl + k0 + cc]) : (rr == cc ? 1.f : 0.f);
                 }
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
@@ -1337,14 +1345,14 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
     // block, rows r0 .. r0 + 63, into the upper triangle of T and split into (uhk, ulk).
     auto panel_tile = [&](int k0, int bs, int c0, int r0, float *uhk, float *ulk) {
         float acc[4][4] = {};
-        gemm64<false, false>(acc, a.Li + (size_t)k0 * ldl + k0, ldl, c0, bs, a.T + k0, n, r0, n, 0, min(bs, c0 + GT),
+        gemm64<false, false>(acc, a.Li + (size_t)k0 * ldl + k0, ldl, c0, bs, a.T + k0, ldl, r0, n, 0, min(bs, c0 + GT),
                              TS);
 #pragma unroll
         for (int u = 0; u < 4; u++)
 #pragma unroll
             for (int v = 0; v < 4; v++) {
                 const int c = c0 + ty + 16 * u, r = r0 + tx + 16 * v;
-                if (c < bs && r < n) a.T[(size_t)(k0 + c) * n + r] = acc[u][v];
+                if (c < bs && r < n) a.T[(size_t)(k0 + c) * ldl + r] = acc[u][v];
                 ST[ty + 16 * u][tx + 16 * v] = acc[u][v];
             }
         __syncthreads();
@@ -1415,11 +1423,11 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
 #pragma unroll
             for (int v = 0; v < 4; v++) {
                 const int rr = ty + 16 * u, cc = tx + 16 * v;
-                dv[u][v] = (rr < bs1 && cc <= rr) ? __ldcg(&a.T[(size_t)(k1 + rr) * n + k1 + cc]) : 0.f;
+                dv[u][v] = (rr < bs1 && cc <= rr) ? __ldcg(&a.T[(size_t)(k1 + rr) * ldl + k1 + cc]) : 0.f;
             }
         for (int e = tid; e < BD * BD; e += PS_THREADS) {
             const int rr = e / BD, m = e % BD;
-            SA[rr][m] = rr < bs1 ? __ldcg(&a.T[(size_t)(k1 + rr) * n + k0 + m]) : 0.f;
+            SA[rr][m] = rr < bs1 ? __ldcg(&a.T[(size_t)(k1 + rr) * ldl + k0 + m]) : 0.f;
         }
         __syncthreads();
         {
@@ -1444,7 +1452,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 for (int v = 0; v < 4; v++) {
                     const int c = ty + 16 * u, r = tx + 16 * v;
                     S0[c][r] = r < bs1 ? acc[u][v] : 0.f;
-                    if (r < bs1) a.T[(size_t)(k0 + c) * n + k1 + r] = acc[u][v];
+                    if (r < bs1) a.T[(size_t)(k0 + c) * ldl + k1 + r] = acc[u][v];
                 }
         }
         __syncthreads();
@@ -1550,21 +1558,19 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                     const int bs1 = min(BD, rest);
                     const int ntt = (rest + TT - 1) / TT, ntiles = ntt * (ntt + 1) / 2;
                     const int ncr = blocked ? 0 : (k1 + TT - 1) / TT, nall = ntiles + ntt * ncr;
-                    for (int t = wid; t < nall; t += W) {
-                        bool ok;
-                        if (t < ntiles) {
-                            int bi, bj;
-                            tri_tile(t, bi, bj);
-                            ok = trailing_tile_tc<BD>(ts, uhk, ulk, uhk, ulk, a.T, n, n, k1 + bi * TT, k1 + bj * TT,
-                                                      t == 0 ? k1 + bs1 : 0, 0);
-                            if (ok && t == 0) flag_set(fl_t, kb + 1);
-                        } else {
+                    auto job = [&](int t) -> TileJob {
+                        if (t >= ntiles) {
                             const int tr = t - ntiles;
-                            ok = trailing_tile_tc<BD>(ts, uhk, ulk, a.xh, a.xl, a.Li, n, ldl, k1 + (tr / ncr) * TT,
-                                                      (tr % ncr) * TT, k0, k1);
+                            return {uhk, ulk, a.xh, a.xl, a.Li, k1 + tr / ncr * TT, tr % ncr * TT, k0, k1};
                         }
-                        if (!ok) return;
-                    }
+                        int bi, bj;
+                        tri_tile(t, bi, bj);
+                        return {uhk, ulk, uhk, ulk, a.T, k1 + bi * TT, k1 + bj * TT, t == 0 ? k1 + bs1 : 0, 0};
+                    };
+                    if (!rank_update_tiles<BD>(ts, n, ldl, wid, W, nall, job, [&](int t) {
+                            if (t == 0) flag_set(fl_t, kb + 1);
+                        }))
+                        return;
                 }
                 if (!grid_barrier(wbar, a.err, W)) return;
             }
@@ -1606,17 +1612,18 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 } else if (bx == 0) {
                     // D -= U_kb^T U_kb on the lower 64 x 64 tiles of the next diagonal block, FP32
                     // from U (= L^T, the upper triangle rows k0 .. k0 + bs - 1 of T)
-                    const float *U = a.T + (size_t)k0 * n;
+                    const float *U = a.T + (size_t)k0 * ldl;
                     for (int ti = 0; ti * GT < bs1; ti++)
                         for (int tj = 0; tj <= ti; tj++) {
                             float acc[4][4] = {};
-                            gemm64<true, true>(acc, U, n, k1 + ti * GT, k1 + bs1, U, n, k1 + tj * GT, k1 + bs1, 0, bs, TS);
+                            gemm64<true, true>(acc, U, ldl, k1 + ti * GT, k1 + bs1, U, ldl, k1 + tj * GT, k1 + bs1, 0, bs,
+                                               TS);
     #pragma unroll
                             for (int u = 0; u < 4; u++)
     #pragma unroll
                                 for (int v = 0; v < 4; v++) {
                                     const int i = k1 + ti * GT + ty + 16 * u, j = k1 + tj * GT + tx + 16 * v;
-                                    if (i < k1 + bs1 && j <= i) a.T[(size_t)i * n + j] -= acc[u][v];
+                                    if (i < k1 + bs1 && j <= i) a.T[(size_t)i * ldl + j] -= acc[u][v];
                                 }
                             __syncthreads();
                         }
@@ -1625,20 +1632,16 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 const int ntt = (rest + TT - 1) / TT, ntiles = ntt * (ntt + 1) / 2;
                 const int ncr = blocked ? 0 : (k1 + TT - 1) / TT, nall = ntiles + ntt * ncr;
                 const int t0 = G > 1 ? bx - 1 : 0, dt = G > 1 ? G - 1 : 1;
-                for (int t = t0; t >= 0 && t < nall; t += dt) {
-                    bool ok;
-                    if (t < ntiles) {
-                        int bi, bj;
-                        tri_tile(t, bi, bj);
-                        ok = trailing_tile_tc<BD>(ts, a.uh, a.ul, a.uh, a.ul, a.T, n, n, k1 + bi * TT, k1 + bj * TT,
-                                                  t == 0 ? k1 + bs1 : 0, 0);
-                    } else {
+                auto job = [&](int t) -> TileJob {
+                    if (t >= ntiles) {
                         const int tr = t - ntiles;
-                        ok = trailing_tile_tc<BD>(ts, a.uh, a.ul, a.xh, a.xl, a.Li, n, ldl, k1 + (tr / ncr) * TT,
-                                                  (tr % ncr) * TT, k0, k1);
+                        return {a.uh, a.ul, a.xh, a.xl, a.Li, k1 + tr / ncr * TT, tr % ncr * TT, k0, k1};
                     }
-                    if (!ok) return;
-                }
+                    int bi, bj;
+                    tri_tile(t, bi, bj);
+                    return {a.uh, a.ul, a.uh, a.ul, a.T, k1 + bi * TT, k1 + bj * TT, t == 0 ? k1 + bs1 : 0, 0};
+                };
+                if (t0 >= 0 && !rank_update_tiles<BD>(ts, n, ldl, t0, dt, nall, job, [](int) {})) return;
             }
             if (!grid_barrier(a.bar, a.err, G)) return;
             if (__ldcg(a.status) >= 0) return;                  // broken factor: every CTA leaves here
@@ -1662,13 +1665,13 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 const int q0 = t / per * 2 * m, i0 = q0 + m + t % per / mt * GT, j0 = q0 + t % mt * GT;
                 if (i0 >= n) continue;
                 float acc[4][4] = {};
-                gemm64<true, true>(acc, a.T, n, i0, n, a.Li, ldl, j0, q0 + m, j0, q0 + m, TS);
+                gemm64<true, true>(acc, a.T, ldl, i0, n, a.Li, ldl, j0, q0 + m, j0, q0 + m, TS);
 #pragma unroll
                 for (int u = 0; u < 4; u++)
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
                         const int i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
-                        if (i < n) a.T[(size_t)i * n + j] = acc[u][v];
+                        if (i < n) a.T[(size_t)i * ldl + j] = acc[u][v];
                     }
             }
             if (!grid_barrier(a.bar, a.err, G)) return;
@@ -1676,7 +1679,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 const int q0 = t / per * 2 * m, i0 = q0 + m + t % per / mt * GT, j0 = q0 + t % mt * GT;
                 if (i0 >= n) continue;
                 float acc[4][4] = {};
-                gemm64<false, true>(acc, a.Li, ldl, i0, n, a.T, n, j0, q0 + m, q0 + m, min(n, i0 + GT), TS);
+                gemm64<false, true>(acc, a.Li, ldl, i0, n, a.T, ldl, j0, q0 + m, q0 + m, min(n, i0 + GT), TS);
 #pragma unroll
                 for (int u = 0; u < 4; u++)
 #pragma unroll
@@ -1931,11 +1934,11 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                     const int c0 = warp * SEG;
                     float acc = 0.f;
                     if (i < n) {
-                        const float *u = a.T + (size_t)(s0 + c0) * n + i;
+                        const float *u = a.T + (size_t)(s0 + c0) * ldl + i;
                         for (int c = 0; c < SEG; c += 32) {
                             float uv[32];
 #pragma unroll
-                            for (int q = 0; q < 32; q++) uv[q] = __ldcg(u + (size_t)(c + q) * n);
+                            for (int q = 0; q < 32; q++) uv[q] = __ldcg(u + (size_t)(c + q) * ldl);
 #pragma unroll
                             for (int q = 0; q < 32; q++) acc = fmaf(uv[q], ys[c0 + c + q], acc);
                         }
@@ -1969,7 +1972,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 for (int r = tid; r < SB; r += PS_THREADS) zs[r] = s0 + r < s1 ? __ldcg(a.rf + s0 + r) : 0.f;
                 __syncthreads();
                 for (int i = gwarp; i < s0; i += gwarps) {
-                    const float *u = a.T + (size_t)i * n;
+                    const float *u = a.T + (size_t)i * ldl;
                     float acc = 0.f;
                     float uv[SB / 32];
 #pragma unroll
@@ -2316,6 +2319,7 @@ static void enqueue_front(MixedWs &w, const MixedPlan &pl, double *O, const doub
     g.shift = (float)shift;
     g.C = w.T.p;
     g.n = pl.n;
+    g.ldc = (pl.n + 31) / 32 * 32;
     g.err = err;
     const int nt = (int)(pl.rows_pad / TC_M);
     g.split = pl.split ? 1 : 0;
@@ -2327,7 +2331,7 @@ static void enqueue_front(MixedWs &w, const MixedPlan &pl, double *O, const doub
             k_gram_tf32_tc<<<dim3(nt * (nt + 1) / 2, 3), 128, TC_SMEM, st>>>(mh, ml, g);
         }
         NQS_LAUNCH("gram_sum");
-        k_gram_sum<<<std::min(pl.n, 65535), 256, 0, st>>>(w.Tp.p, pl.n, g.scale, g.shift, w.T.p);
+        k_gram_sum<<<std::min(pl.n, 65535), 256, 0, st>>>(w.Tp.p, pl.n, g.ldc, g.scale, g.shift, w.T.p);
     } else {
         NQS_LAUNCH("gram_tc");
         k_gram_tf32_tc<<<nt * (nt + 1) / 2, 128, TC_SMEM, st>>>(mh, ml, g);
@@ -2430,7 +2434,7 @@ static bool prepare_ws(MixedWs &w, const MixedPlan &pl, int Ns, long P, cudaStre
     // split U^T: a trailing tile starting at row k1 + 128 bi reaches row n + 126 at most; pad rows read as zero.
     // Sized for the wide diagonal block so a batch's autotuner can pick either width.
     const size_t nu = (size_t)(n + TT) * BD_LARGE;
-    if (!w.T.ensure((size_t)n * n) || !w.Li.ensure((size_t)n * ldl) || !w.LiT.ensure((size_t)n * ldl) ||
+    if (!w.T.ensure((size_t)n * ldl) || !w.Li.ensure((size_t)n * ldl) || !w.LiT.ensure((size_t)n * ldl) ||
         !w.rf.ensure(ldl) || !w.zf.ensure(ldl) || !w.rhs.ensure(n) || !w.r.ensure(n) || !w.r2.ensure(n) ||
         !w.u.ensure(big) ||
         !w.p.ensure(n) || !w.q.ensure(n) || !w.z.ensure(n) || !w.uh.ensure(nu) || !w.ul.ensure(nu) ||
@@ -3110,7 +3114,7 @@ int nqs_gpu_gram_tc(const double *O_host, int Ns, long P, int passes, double sca
     g.scale = (float)scale;
     g.shift = 0.f;
     g.C = w.T.p;
-    g.n = Ns;
+    g.n = g.ldc = Ns;
     g.err = err.p;
     g.split = 0;
     if (!NQS_CUDA(cudaFuncSetAttribute(k_gram_tf32_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM)))
