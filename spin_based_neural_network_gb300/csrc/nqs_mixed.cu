@@ -341,128 +341,6 @@ __device__ __forceinline__ unsigned long long gtimer() {
     return t;
 }
 
-// Factor the 128 x 128 block in S (rows >= bs padded with the identity) in four
-// 32-column sub-panels and leave the inverses of the four diagonal 32 x 32
-// factors in the matching diagonal blocks of X.  The 32 x 32 factor and its
-// inverse run in one warp's registers; the panel below it and the update of the
-// rest of the block use the whole CTA.  Returns the first failing column or -1.
-template <int BD>
-__device__ int block_chol(float (*S)[BT + 1], float (*X)[BT + 1], int bs, int *s_flag, float *tmp) {
-    constexpr int NSUB = BD / 32;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int e = tid; e < BD * BD; e += PS_THREADS) X[e / BD][e % BD] = 0.f;
-    for (int sb = 0; sb < NSUB; sb++) {
-        const int c0 = sb * 32;
-        if (warp == 0) {
-            // right-looking, lane = row in registers; the scaled column j is
-            // broadcast through shared memory (a shuffle per entry is ~3x slower)
-            // Lane = row; column j of L is broadcast by shuffles.  Branch-free:
-            // every lane updates its whole row, and the entries right of a lane's
-            // diagonal (zero on entry) become scratch that nothing reads (lane i's
-            // row[c], c > i, is only broadcast at steps j = c > i, which read lanes
-            // c' > j only).  A non-positive pivot records the first failing column
-            // and continues on a unit pivot; the block is discarded then.  (With
-            // a per-entry `c <= lane` guard this loop ran ~4x slower.)
-            float row[32];
-#pragma unroll
-            for (int c = 0; c < 32; c++) row[c] = S[c0 + lane][c0 + c];
-            int fail = -1;
-            float dinv = 0.f;                                  // lane j keeps 1 / L_jj
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const float d = __shfl_sync(0xffffffffu, row[j], j);
-                const bool ok = d > 0.f;
-                fail = (fail < 0 && !ok) ? j : fail;
-                const float inv = rsqrtf(ok ? d : 1.f);
-                row[j] *= inv;                                 // lane j: d / sqrt(d) = L_jj
-                dinv = lane == j ? inv : dinv;
-                const float lrj = row[j];                     // L[lane][j]
-#pragma unroll
-                for (int c = j + 1; c < 32; c++) row[c] = fmaf(-lrj, __shfl_sync(0xffffffffu, lrj, c), row[c]);
-            }
-#pragma unroll
-            for (int c = 0; c < 32; c++)
-                if (c <= lane) S[c0 + lane][c0 + c] = row[c];
-            if (lane == 0) *s_flag = (fail >= 0 && c0 + fail < bs) ? c0 + fail : -1;
-            __syncwarp();
-            if (fail < 0) {
-                // X_s = L_s^{-1} by forward substitution, lane = column
-                float x[32];
-#pragma unroll
-                for (int rr = 0; rr < 32; rr++) {
-                    const float di = __shfl_sync(0xffffffffu, dinv, rr);
-                    float s0 = (rr == lane) ? 1.f : 0.f, s1 = 0.f;
-#pragma unroll
-                    for (int m = 0; m < rr; m += 2) {
-                        s0 -= S[c0 + rr][c0 + m] * x[m];
-                        if (m + 1 < rr) s1 -= S[c0 + rr][c0 + m + 1] * x[m + 1];
-                    }
-                    x[rr] = rr < lane ? 0.f : (s0 + s1) * di;
-                }
-#pragma unroll
-                for (int rr = 0; rr < 32; rr++) X[c0 + rr][c0 + lane] = x[rr];
-            }
-        }
-        __syncthreads();
-        if (*s_flag >= 0) return *s_flag;
-        const int t0 = c0 + 32, nr = BD - t0;
-        if (nr == 0) break;
-        // rows below the sub-panel: L[r][c0+j] = sum_m A[r][c0+m] X_s[j][m]
-        for (int w = tid; w < nr * 8; w += PS_THREADS) {
-            const int r = t0 + w / 8, j0 = (w % 8) * 4;
-            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll 8
-            for (int m = 0; m < 32; m++) {
-                float av = S[r][c0 + m];
-                a0 += av * X[c0 + j0][c0 + m];
-                a1 += av * X[c0 + j0 + 1][c0 + m];
-                a2 += av * X[c0 + j0 + 2][c0 + m];
-                a3 += av * X[c0 + j0 + 3][c0 + m];
-            }
-            tmp[w * 4 + 0] = a0;
-            tmp[w * 4 + 1] = a1;
-            tmp[w * 4 + 2] = a2;
-            tmp[w * 4 + 3] = a3;
-        }
-        __syncthreads();
-        for (int w = tid; w < nr * 8; w += PS_THREADS) {
-            const int r = t0 + w / 8, j0 = (w % 8) * 4;
-#pragma unroll
-            for (int q = 0; q < 4; q++) S[r][c0 + j0 + q] = tmp[w * 4 + q];
-        }
-        __syncthreads();
-        // rest of the block: S[i][j] -= sum_m L[i][c0+m] L[j][c0+m], 4 x 4 outputs
-        // per thread on rows / columns strided by nr / 4
-        const int q = nr / 4;
-        for (int e = tid; e < q * q; e += PS_THREADS) {
-            const int ti = e / q, tj = e % q;
-            float acc[4][4] = {};
-#pragma unroll 4
-            for (int m = 0; m < 32; m++) {
-                float av[4], bv[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    av[u] = S[t0 + ti + q * u][c0 + m];
-                    bv[u] = S[t0 + tj + q * u][c0 + m];
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int v = 0; v < 4; v++) acc[u][v] = fmaf(av[u], bv[v], acc[u][v]);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) {
-                    const int i = t0 + ti + q * u, j = t0 + tj + q * v;
-                    if (j <= i) S[i][j] -= acc[u][v];
-                }
-        }
-        __syncthreads();
-    }
-    return -1;
-}
-
 // The 64 x 64 diagonal block, Cholesky and X = L^{-1} in one right-looking sweep over
 // four-column panels with the block in registers: thread (w, l) = (tid / 32, tid % 32)
 // holds rows i = w + 8u (u < 8) and columns c = l + 32v (v < 2) of S and of
@@ -627,61 +505,78 @@ __device__ int block_chol_inv64(const float (*S)[BT + 1], float (*X)[BT + 1], in
     return fail;
 }
 
-// Off-diagonal 32-blocks of X = L^{-1} inside the 128-block (the diagonal
-// 32-blocks are already in X): for d = 1..3, X_ba = -X_bb (sum_{m=a}^{b-1}
-// L_bm X_ma), b = a + d, all pairs of one block diagonal computed by the CTA,
-// 4 x 4 outputs per thread (rows and columns strided by 8).
-template <int BD>
-__device__ void block_inv(float (*S)[BT + 1], float (*X)[BT + 1], float *tmp) {
-    constexpr int NSUB = BD / 32;
-    const int tid = threadIdx.x, r8 = (tid >> 3) & 7, c8 = tid & 7;
-    for (int d = 1; d < NSUB; d++) {
-        const int pairs = NSUB - d;
-        for (int w = tid; w < pairs * 64; w += PS_THREADS) {
-            const int pa = w >> 6, ob = (pa + d) * 32, oa = pa * 32;
-            float acc[4][4] = {};
-#pragma unroll 4
-            for (int m = oa; m < ob; m++) {
-                float sv[4], xv[4];
+// 64 x 64 products of shared-memory blocks (pitch BT + 1), 4 x 4 entries a thread (rows ty + 16u,
+// columns tx + 16v): acc += sum_m A[row][m] B[col][m] (BT_ROWS) or sum_m A[row][m] B[m][col].
+template <bool BT_ROWS>
+__device__ __forceinline__ void smem_product64(float (&acc)[4][4], const float (*A)[BT + 1], const float (*B)[BT + 1]) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 8
+    for (int m = 0; m < 64; m++) {
+        float a[4], b[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    sv[u] = S[ob + r8 + 8 * u][m];
-                    xv[u] = X[m][oa + c8 + 8 * u];
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int v = 0; v < 4; v++) acc[u][v] = fmaf(sv[u], xv[v], acc[u][v]);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) tmp[pa * 1024 + (r8 + 8 * u) * 32 + c8 + 8 * v] = acc[u][v];
+        for (int u = 0; u < 4; u++) {
+            a[u] = A[ty + 16 * u][m];
+            b[u] = BT_ROWS ? B[tx + 16 * u][m] : B[m][tx + 16 * u];
         }
-        __syncthreads();
-        for (int w = tid; w < pairs * 64; w += PS_THREADS) {
-            const int pa = w >> 6, ob = (pa + d) * 32, oa = pa * 32;
-            float acc[4][4] = {};
-#pragma unroll 4
-            for (int m = 0; m < 32; m++) {              // X_bb is lower triangular (zeros above)
-                float xv[4], tv[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    xv[u] = X[ob + r8 + 8 * u][ob + m];
-                    tv[u] = tmp[pa * 1024 + m * 32 + c8 + 8 * u];
-                }
+        for (int u = 0; u < 4; u++)
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int v = 0; v < 4; v++) acc[u][v] = fmaf(xv[u], tv[v], acc[u][v]);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) X[ob + r8 + 8 * u][oa + c8 + 8 * v] = -acc[u][v];
-        }
-        __syncthreads();
+            for (int v = 0; v < 4; v++) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
     }
+}
+
+// The 128 x 128 diagonal block in two 64-wide sweeps: X11 of S11, L21 = S21 X11^T, S22 - L21 L21^T,
+// X22 of that, X21 = -X22 (L21 X11).  S (rows >= bs padded with the identity) is overwritten; X gets
+// L^{-1} with zeros above the diagonal.  Returns the first non-positive pivot column below bs or -1.
+// Measured: MEAS_B128 us a block, 46 us in four 32-wide sub-panels.
+__device__ int block_chol_inv128(float (*S)[BT + 1], float (*X)[BT + 1], int bs, float *buf) {
+    typedef float (*Block)[BT + 1];
+    const Block S21 = (Block)&S[64][0], S22 = (Block)&S[64][64], X12 = (Block)&X[0][64], X21 = (Block)&X[64][0],
+                X22 = (Block)&X[64][64];
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    int f = block_chol_inv64(S, X, min(bs, 64), buf);
+    if (f >= 0) return f;
+    __syncthreads();
+    float acc[4][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) acc[u][v] = 0.f;
+    };
+    auto put = [&](Block D, float sign) {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) D[ty + 16 * u][tx + 16 * v] = sign * acc[u][v];
+    };
+    clear();
+    smem_product64<true>(acc, S21, X);                      // L21[r][c] = sum_m S21[r][m] X11[c][m]
+    __syncthreads();
+    put(S21, 1.f);
+    __syncthreads();
+    clear();
+    smem_product64<true>(acc, S21, S21);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int v = 0; v < 4; v++) S22[ty + 16 * u][tx + 16 * v] -= acc[u][v];
+    __syncthreads();
+    f = block_chol_inv64(S22, X22, max(bs - 64, 0), buf);
+    if (f >= 0) return 64 + f;
+    __syncthreads();
+    clear();
+    smem_product64<false>(acc, S21, X);                     // W = L21 X11
+    put(X12, 1.f);
+    __syncthreads();
+    clear();
+    smem_product64<false>(acc, X22, X12);
+    put(X21, -1.f);
+    __syncthreads();
+    clear();
+    put(X12, 1.f);
+    __syncthreads();
+    return -1;
 }
 
 // GEMM tile: acc[u][v] += sum_{m in [kb, ke)} A(r0 + ty + 16u, m) B(c0 + tx + 16v, m)
@@ -991,8 +886,9 @@ __device__ __forceinline__ void stage_sw128(uint32_t sbase, const float *X, int 
 
 struct TcState {
     uint8_t *sm;          // 2 stages of TT_STAGE_BYTES, 1024-byte aligned, and a 128 x 132 tile of T
-    uint64_t *mbar;       // [2] MMA completion per stage
+    uint64_t *mbar;       // [2] MMA completion per stage; [2] TMA arrival per stage, [1] of the tile of T
     uint32_t cnt[2];      // commits issued per stage (mbarrier phase tracking)
+    uint32_t tma[3];      // TMA loads waited for, per barrier mbar[2 ..]
     uint32_t tmem;        // 128 TMEM columns (128 x 128 FP32 accumulator)
     int *err;
 };
@@ -1139,6 +1035,164 @@ __device__ __forceinline__ bool rank_update_tiles(TcState &ts, int n, int ldt, i
     return true;
 }
 
+// Trailing tiles of the 128-wide factor of a large system (mode lim == 0 of rank_update_tiles) with the
+// operands and the tiles of T brought by TMA, so that no thread spends its time issuing copies: thread
+// 0 runs the operand ring and the MMAs of tile t while warps 1 .. 7 store tile t - 1 and thread 32 then
+// brings T's values of tile t into the freed buffer (four 32-column boxes, 128-byte swizzle); the
+// update in shared memory joins the two.  Rows past n arrive as zeros and are not stored.
+// mu: tensor maps of U^T's hi and lo words ([row][128]) and of T.  The tiles' rows R0 = k1 + 128 bi and
+// columns C0 = k1 + 128 bj are multiples of 128, as every box start has to be of 16 bytes.
+// Measured, order 15014: MEAS_TT a tile, 8 us with the copies issued by the threads (16 bytes a lane:
+// 64 bytes a clock and SM through the load path, 10 k of the 16 k clocks of a tile).
+__device__ __forceinline__ void proxy_fence_global() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Waits for a TMA load already issued, whatever the error word says (before its buffer is given up).
+__device__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+    for (uint32_t it = 0; it < (1u << 24) && !mbar_try_wait(bar, parity); it++)
+        if (it > 256) __nanosleep(64);
+}
+
+__device__ __forceinline__ bool trailing_tiles_tma(TcState &ts, const CUtensorMap *mu, float *T, int n, int ldt, int k1,
+                                                   int t0, int dt, int nall) {
+    if (t0 >= nall) return true;
+    constexpr int NQ = BD_LARGE / 32, SUB = TT * 32 * 4;     // SUB: bytes of a 32-column box of T
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t *const tb = ts.sm + 2 * TT_STAGE_BYTES;
+    uint64_t *const mma = ts.mbar, *const full = ts.mbar + 2, *const tfull = ts.mbar + 4;
+    const uint32_t s0 = smem_u32(ts.sm);
+    const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TT >> 3) << 17) | ((uint32_t)(TT >> 4) << 24);
+    auto place = [&](int t, int &R0, int &C0) {
+        int bi, bj;
+        tri_tile(t, bi, bj);
+        R0 = k1 + bi * TT;
+        C0 = k1 + bj * TT;
+    };
+    auto load = [&](int R0, int C0, int q) {                 // thread 0: chunk q; one side when the tile is diagonal
+        uint8_t *sb = ts.sm + (q & 1) * TT_STAGE_BYTES;
+        mbar_expect_tx(&full[q & 1], (R0 == C0 ? 2 : 4) * TT_CHUNK_BYTES);
+        tma_load_2d(sb, mu, &full[q & 1], q * 32, R0);
+        tma_load_2d(sb + TT_CHUNK_BYTES, mu + 1, &full[q & 1], q * 32, R0);
+        if (R0 != C0) {
+            tma_load_2d(sb + 2 * TT_CHUNK_BYTES, mu, &full[q & 1], q * 32, C0);
+            tma_load_2d(sb + 3 * TT_CHUNK_BYTES, mu + 1, &full[q & 1], q * 32, C0);
+        }
+    };
+    // 16-byte slot c (of 8) of row r in box b
+    auto slot = [&](int b, int r, int c) { return (float4 *)(tb + b * SUB + r * 128 + ((c ^ (r & 7)) << 4)); };
+    auto store = [&](int t, int thread, int threads) {
+        int R0, C0;
+        place(t, R0, C0);
+        for (int e = thread; e < TT * 32; e += threads) {
+            const int r = e >> 5, c = e & 31, i = R0 + r, j = C0 + 4 * c;
+            if (i >= n || j > i) continue;
+            const float4 o = *slot(c >> 3, r, c & 7);
+            float *d = &T[(size_t)i * ldt + j];
+            if (j + 3 <= i) {
+                *(float4 *)d = o;
+            } else {                                         // the diagonal crosses this group
+                d[0] = o.x;
+                if (j + 1 <= i) d[1] = o.y;
+                if (j + 2 <= i) d[2] = o.z;
+            }
+        }
+    };
+    int R0, C0;
+    place(t0, R0, C0);
+    uint32_t issued[2] = {ts.tma[0], ts.tma[1]};             // thread 0: loads issued per stage
+    if (tid == 0) {
+        proxy_fence_global();                                // the panel's writes, acquired at the barrier
+        for (int q = 0; q < 2; q++, issued[q - 1]++) load(R0, C0, q);
+    }
+    if (tid == 32) proxy_fence_global();
+    for (int t = t0; t < nall; t += dt) {
+        bool ok = true;
+        if (warp == 0) {
+            if (lane == 0) {
+                const bool diag = R0 == C0;
+                for (int q = 0; q < NQ && ok; q++) {
+                    const int b = q & 1;
+                    ok = mbar_wait(&full[b], ts.tma[b] & 1, ts.err);
+                    if (!ok) break;
+                    ts.tma[b]++;
+                    tc_fence_after();
+                    const uint32_t sa = s0 + b * TT_STAGE_BYTES, sb = diag ? sa : sa + 2 * TT_CHUNK_BYTES;
+#pragma unroll
+                    for (int pass = 0; pass < 3; pass++) {   // hi hi, hi lo, lo hi
+                        const uint32_t pa = sa + (pass == 2 ? TT_CHUNK_BYTES : 0);
+                        const uint32_t pb = sb + (pass == 1 ? TT_CHUNK_BYTES : 0);
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            umma_tf32(ts.tmem, sw128_desc(pa + k * 32), sw128_desc(pb + k * 32), idesc,
+                                      (q | pass | k) ? 1u : 0u);
+                    }
+                    umma_commit(&mma[b]);
+                    ts.cnt[b]++;
+                    if (q >= 1 && q + 1 < NQ) {
+                        ok = mbar_wait(&mma[b ^ 1], (ts.cnt[b ^ 1] - 1) & 1, ts.err);
+                        if (ok) {
+                            load(R0, C0, q + 1);
+                            issued[b ^ 1]++;
+                        }
+                    }
+                }
+                ok = ok && mbar_wait(&mma[1], (ts.cnt[1] - 1) & 1, ts.err) &&
+                     mbar_wait(&mma[0], (ts.cnt[0] - 1) & 1, ts.err);
+                if (ok && t + dt < nall) {
+                    int Rn, Cn;
+                    place(t + dt, Rn, Cn);
+                    for (int q = 0; q < 2; q++, issued[q - 1]++) load(Rn, Cn, q);
+                }
+            }
+            __syncwarp();
+        } else {
+            if (t != t0) store(t - dt, tid - 32, PS_THREADS - 32);
+            asm volatile("bar.sync 1, 224;" ::: "memory");
+            if (tid == 32) {
+                mbar_expect_tx(tfull, 4 * SUB);
+                for (int b = 0; b < 4; b++) tma_load_2d(tb + b * SUB, mu + 2, tfull, C0 + 32 * b, R0);
+            }
+        }
+        ok = __syncthreads_and(ok);
+        ok = ok && mbar_wait(tfull, ts.tma[2] & 1, ts.err);
+        if (!__syncthreads_and(ok)) {                        // given up: own copies and MMAs land first
+            mbar_drain(tfull, ts.tma[2] & 1);
+            if (tid == 0)
+                for (int b = 0; b < 2; b++) {
+                    for (; ts.tma[b] < issued[b]; ts.tma[b]++) mbar_drain(&full[b], ts.tma[b] & 1);
+                    if (ts.cnt[b] > 0) mbar_drain(&mma[b], (ts.cnt[b] - 1) & 1);
+                }
+            __syncthreads();
+            return false;
+        }
+        ts.tma[2]++;
+        tc_fence_after();
+        const int row = 32 * (warp & 3) + lane;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int b = 2 * (warp >> 2) + h;
+            float v[32];
+            tmem_ld32(ts.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * b), v);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                float4 *p = slot(b, row, j);
+                float4 o = *p;
+                o.x -= v[4 * j];
+                o.y -= v[4 * j + 1];
+                o.z -= v[4 * j + 2];
+                o.w -= v[4 * j + 3];
+                *p = o;
+            }
+        }
+        tc_fence_before();
+        fence_proxy_async();                                 // tb is written by TMA next
+        __syncthreads();
+        if (t + dt < nall) place(t + dt, R0, C0);
+        else store(t, tid, PS_THREADS);
+    }
+    __syncthreads();
+    return true;
+}
+
 // Order from which the preconditioner is applied by blocked substitution
 // instead of through an explicit L^{-1}.
 constexpr int BLOCKED_SOLVE_MIN = 4608;
@@ -1186,7 +1240,8 @@ struct FrArgs {
 // (all co-resident): the whole grid for a single system, a slice of it when a
 // batch of systems shares one launch.
 template <int BD>
-__device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int G, TcState &ts) {
+__device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int G, TcState &ts,
+                                        const CUtensorMap *mu = nullptr) {
     extern __shared__ float psm[];
     float (*S0)[BT + 1] = (float (*)[BT + 1])psm;
     float (*S1)[BT + 1] = (float (*)[BT + 1])(psm + BT * (BT + 1));
@@ -1197,7 +1252,6 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
     const int gtid = bx * PS_THREADS + tid, gthreads = G * PS_THREADS;
     const int gwarp = bx * (PS_THREADS / 32) + (tid >> 5), gwarps = G * (PS_THREADS / 32);
     const int nb = (n + BD - 1) / BD;
-    __shared__ int s_flag;
     __shared__ float tmpb[3 * 1024];
     unsigned long long tacc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const bool timing = a.tm != nullptr && bx == 0 && tid == 0;
@@ -1253,8 +1307,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 }
             }
             __syncthreads();
-            f = block_chol<BD>(S0, S1, bs, &s_flag, tmpb);
-            if (f < 0) block_inv<BD>(S0, S1, tmpb);
+            f = block_chol_inv128(S0, S1, bs, tmpb);
         }
         if (f >= 0) {
             if (tid == 0) {
@@ -1277,6 +1330,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
     // preconditioner by substitution over SB-wide blocks (two grid barriers per block and
     // direction); below BLOCKED_SOLVE_MIN the inverse is built beside the factor.
     const bool blocked = n >= BLOCKED_SOLVE_MIN;
+    const bool tma_tiles = BD == BD_LARGE && blocked && mu != nullptr;
     // X = L^{-1} is built beside the factor (forward substitution of L X = I, right-looking
     // by block columns): R = I - sum_{p < kb} L_{:,p} X_{p,:} accumulates in the lower
     // off-diagonal blocks of Li.  In the panel phase of step kb block row kb of X is
@@ -1600,6 +1654,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                     if (c0 >= bs) continue;
                     panel_tile(k0, bs, c0, r0, a.uh, a.ul);
                 }
+                if (tma_tiles) proxy_fence_global();            // U^T is read by TMA next
             }
             if (!grid_barrier(a.bar, a.err, G)) return;
             NQS_PHASE(1);
@@ -1607,7 +1662,11 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
             // the update of R by block row kb of X
             {
                 const int bs1 = min(BD, rest);                  // order of the next diagonal block
-                if (bx == 0 && BD == 64) {
+                if (bx == 0 && tma_tiles) {
+                    // trailing tile 0 is the next diagonal block
+                    if (!trailing_tiles_tma(ts, mu, a.T, n, ldl, k1, 0, 1, 1)) return;
+                    factor_diag(kb + 1, -1, 0);
+                } else if (bx == 0 && BD == 64) {
                     factor_diag(kb + 1, k0, bs);                // the update fused into the block's load
                 } else if (bx == 0) {
                     // D -= U_kb^T U_kb on the lower 64 x 64 tiles of the next diagonal block, FP32
@@ -1631,7 +1690,8 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 }
                 const int ntt = (rest + TT - 1) / TT, ntiles = ntt * (ntt + 1) / 2;
                 const int ncr = blocked ? 0 : (k1 + TT - 1) / TT, nall = ntiles + ntt * ncr;
-                const int t0 = G > 1 ? bx - 1 : 0, dt = G > 1 ? G - 1 : 1;
+                // (from tile 1 when CTA 0 has taken tile 0)
+                const int t0 = (G > 1 ? bx - 1 : 0) + (tma_tiles && (bx > 0 || G == 1) ? 1 : 0), dt = G > 1 ? G - 1 : 1;
                 auto job = [&](int t) -> TileJob {
                     if (t >= ntiles) {
                         const int tr = t - ntiles;
@@ -1641,7 +1701,12 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                     tri_tile(t, bi, bj);
                     return {a.uh, a.ul, a.uh, a.ul, a.T, k1 + bi * TT, k1 + bj * TT, t == 0 ? k1 + bs1 : 0, 0};
                 };
-                if (t0 >= 0 && !rank_update_tiles<BD>(ts, n, ldl, t0, dt, nall, job, [](int) {})) return;
+                if (t0 >= 0) {
+                    if (tma_tiles ? !trailing_tiles_tma(ts, mu, a.T, n, ldl, k1, t0, dt, ntiles)
+                                  : !rank_update_tiles<BD>(ts, n, ldl, t0, dt, nall, job, [](int) {}))
+                        return;
+                }
+                if (tma_tiles) proxy_fence_global();            // T is read by TMA next
             }
             if (!grid_barrier(a.bar, a.err, G)) return;
             if (__ldcg(a.status) >= 0) return;                  // broken factor: every CTA leaves here
@@ -2167,10 +2232,10 @@ __device__ __forceinline__ void tc_setup(TcState &ts, uint64_t *mbar, uint32_t *
     ts.sm = (uint8_t *)psm + (((base + 1023u) & ~1023u) - base);
     ts.mbar = mbar;
     ts.cnt[0] = ts.cnt[1] = 0;
+    ts.tma[0] = ts.tma[1] = ts.tma[2] = 0;
     ts.err = err;
     if (threadIdx.x == 0) {
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
+        for (int k = 0; k < 5; k++) mbar_init(&mbar[k], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < 32) {
@@ -2192,12 +2257,18 @@ __device__ __forceinline__ void tc_teardown(const TcState &ts) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(ts.tmem), "r"(TT) : "memory");
 }
 
-__global__ void __launch_bounds__(PS_THREADS, 1) k_factor_refine(FrArgs a) {
-    __shared__ uint64_t mbar[2];
+// Tensor maps of a large system's trailing tiles: U^T hi, U^T lo, T.
+struct FrMaps {
+    CUtensorMap m[3];
+};
+
+__global__ void __launch_bounds__(PS_THREADS, 1) k_factor_refine(FrArgs a, const __grid_constant__ FrMaps maps,
+                                                                int have_maps) {
+    __shared__ uint64_t mbar[5];
     __shared__ uint32_t slot;
     TcState ts;
     tc_setup(ts, mbar, &slot, a.err);
-    if (a.bd == BD_LARGE) fr_body<BD_LARGE>(a, blockIdx.x, gridDim.x, ts);
+    if (a.bd == BD_LARGE) fr_body<BD_LARGE>(a, blockIdx.x, gridDim.x, ts, have_maps ? maps.m : nullptr);
     else fr_body<BD_SMALL>(a, blockIdx.x, gridDim.x, ts);
     tc_teardown(ts);
 }
@@ -2211,7 +2282,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_factor_refine_batch(const FrA
                                                                        const int *__restrict__ nctas) {
     const int i = cta_sys[blockIdx.x];
     const FrArgs a = sys[i];
-    __shared__ uint64_t mbar[2];
+    __shared__ uint64_t mbar[5];
     __shared__ uint32_t slot;
     TcState ts;
     tc_setup(ts, mbar, &slot, a.err);
@@ -2407,8 +2478,11 @@ static void enqueue_mixed(const MixedPlan &pl, double *O, const double *gm, cons
     lc.attrs = at;
     lc.numAttrs = 1;
     {
+        FrMaps maps;
+        const int have = fa.bd == BD_LARGE && make_map(&maps.m[0], w.uh.p, fa.n + TT, BD_LARGE) &&
+                         make_map(&maps.m[1], w.ul.p, fa.n + TT, BD_LARGE) && make_map(&maps.m[2], w.T.p, fa.n, fa.ldl);
         NQS_LAUNCH("factor_refine");
-        cudaLaunchKernelEx(&lc, k_factor_refine, fa);
+        cudaLaunchKernelEx(&lc, k_factor_refine, fa, maps, have);
     }
 }
 
