@@ -528,7 +528,7 @@ __device__ __forceinline__ void smem_product64(float (&acc)[4][4], const float (
 // The 128 x 128 diagonal block in two 64-wide sweeps: X11 of S11, L21 = S21 X11^T, S22 - L21 L21^T,
 // X22 of that, X21 = -X22 (L21 X11).  S (rows >= bs padded with the identity) is overwritten; X gets
 // L^{-1} with zeros above the diagonal.  Returns the first non-positive pivot column below bs or -1.
-// Measured: MEAS_B128 us a block, 46 us in four 32-wide sub-panels.
+// Measured: 42 us a block with its loads and stores; four 32-wide sub-panels took 46 us.
 __device__ int block_chol_inv128(float (*S)[BT + 1], float (*X)[BT + 1], int bs, float *buf) {
     typedef float (*Block)[BT + 1];
     const Block S21 = (Block)&S[64][0], S22 = (Block)&S[64][64], X12 = (Block)&X[0][64], X21 = (Block)&X[64][0],
@@ -911,7 +911,7 @@ struct TileJob {
 // (fetched beside its MMAs into a tile of their own in shared memory) are updated and stored, the
 // first two K chunks of the next tile are in flight.  Bound by the bytes an SM takes from L2 (320 KB a
 // tile at BD = 128, about 60 bytes a clock) rather than by the MMAs.  Measured, order 15014:
-// MEAS_RU a tile; with every tile on its own (operands, then T, then stores) 13 us.  Returns false
+// 9.2 us a tile; with every tile on its own (operands, then T, then stores) 13.5 us.  Returns false
 // when a bounded wait gave up (err raised).
 template <int BD, typename Job, typename Done>
 __device__ __forceinline__ bool rank_update_tiles(TcState &ts, int n, int ldt, int t0, int dt, int nall, Job job,
@@ -1042,7 +1042,7 @@ __device__ __forceinline__ bool rank_update_tiles(TcState &ts, int n, int ldt, i
 // update in shared memory joins the two.  Rows past n arrive as zeros and are not stored.
 // mu: tensor maps of U^T's hi and lo words ([row][128]) and of T.  The tiles' rows R0 = k1 + 128 bi and
 // columns C0 = k1 + 128 bj are multiples of 128, as every box start has to be of 16 bytes.
-// Measured, order 15014: MEAS_TT a tile, 8 us with the copies issued by the threads (16 bytes a lane:
+// Measured, order 15014: 6.7 us a tile, 9.2 us with the copies issued by the threads (16 bytes a lane:
 // 64 bytes a clock and SM through the load path, 10 k of the 16 k clocks of a tile).
 __device__ __forceinline__ void proxy_fence_global() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
