@@ -2,9 +2,9 @@
 //
 // The memory-lean projecting Lanczos over the full 2^N basis (N <= 30):
 //   w = H v                     k_heis_matvec   (bond masks, one state per thread)
-//   w -= alpha v + beta v_prev  k_lz_orth       (alpha reduced from the matvec partials)
+//   w -= alpha v + beta v_prev  k_lz_orth       (alpha from the matvec's grid sum)
 //   w = P w                     k_perm_sum x1-4 (sector projector, nibble bit-permute tables)
-//   v_next = w / ||w||          k_lz_scale      (beta reduced from the projector partials)
+//   v_next = w / ||w||          k_lz_scale      (beta from the projector's grid sum)
 // with the host holding only the tridiagonal (alpha, beta) and its lowest Ritz value.
 //
 // Upstream interfaces replaced:
@@ -49,41 +49,60 @@ struct Bonds {
     unsigned m[ED_MAX_BONDS];
 };
 
-__device__ __forceinline__ double warp_sum_d(double v) {
+// Where a kernel leaves a grid-wide sum: block partials, ticket (zero between launches), result.
+struct GridSum {
+    double *part = nullptr;
+    unsigned *ticket = nullptr;
+    double *out = nullptr;
+};
+
+// Sum over the block in a fixed order (thread 0 holds it): the tree of each warp's values (lane l
+// takes lane l + 16, 8, 4, 2, 1), then the warps in turn.  One warp forms the trees of all eight from
+// shared memory, 9 FP64 instructions where a shuffle tree in every warp takes 40.
+__device__ __forceinline__ double block_sum(double v) {
+    __shared__ double red[2][ED_THREADS];
+    red[0][threadIdx.x] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x < 32) {
+        int in = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
+        for (int half = 16; half > 0; half >>= 1, in ^= 1) {
+            for (int e = threadIdx.x; e < half * (ED_THREADS / 32); e += 32) {
+                const double *p = red[in] + e / half * (2 * half) + e % half;
+                red[in ^ 1][e] = p[0] + p[half];
+            }
+            __syncwarp();
+        }
+        if (threadIdx.x == 0)
+            for (int w = 0; w < ED_THREADS / 32; w++) t += red[in][w];
+    }
+    return t;
 }
 
-// Block sum in a fixed order, stored by thread 0 at part[blockIdx.x].
-__device__ __forceinline__ void block_store(double v, double *part) {
-    __shared__ double red[ED_THREADS / 32];
-    v = warp_sum_d(v);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
+// Grid sum in a fixed order: block partials in part, summed by the last block to finish, whose
+// thread 0 calls fin(total).  So the kernels that use the sum read one number instead of every
+// block summing all partials (at 2^18 states that, with its square root and division in every
+// warp, was most of their time).  *ticket is zero before the first launch and again after each.
+template <typename F>
+__device__ __forceinline__ void grid_sum(double v, double *part, unsigned *ticket, F fin) {
+    __shared__ bool last;
+    v = block_sum(v);
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < ED_THREADS / 32; w++) t += red[w];
-        part[blockIdx.x] = t;
-    }
-}
-
-// Sum of np block partials in a fixed order, returned to every thread of the block.
-__device__ __forceinline__ double block_total(const double *part, int np) {
-    __shared__ double red[ED_THREADS / 32];
-    __shared__ double tot;
-    double v = 0.0;
-    for (int i = threadIdx.x; i < np; i += ED_THREADS) v += part[i];
-    v = warp_sum_d(v);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < ED_THREADS / 32; w++) t += red[w];
-        tot = t;
+        part[blockIdx.x] = v;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    return tot;
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += ED_THREADS) t += __ldcg(part + i);
+    t = block_sum(t);
+    if (threadIdx.x == 0) {
+        *ticket = 0;
+        fin(t);
+    }
 }
 
 // y = H x, H = J sum_b S_u.S_v: diagonal J/4 (nb - 2 n_anti) (a table indexed by n_anti),
@@ -92,12 +111,13 @@ __device__ __forceinline__ double block_total(const double *part, int np) {
 // 256-byte segment.  GB300 issues an FP64 add for a whole warp at 16 cycles whatever its
 // active lanes, so the bonds away from the lane bits -- where all 32 states of the warp
 // agree -- are first collected into a warp-uniform bit mask and only the antiparallel ones
-// are loaded (four at a time) and added.  part (may be null) receives the block partials
-// of x.y.  popc >= 0 restricts to the states with that many set bits (down spins): the
-// others are written as 0 without being evaluated.
+// are loaded (four at a time) and added; of the lane-bit bonds each lane takes its own
+// antiparallel ones in turn (the warp adds as often as its busiest lane has bonds, about 12 of 18
+// at N = 18).  R.part (may be null) takes the grid sum of x.y to *R.out.  popc >= 0 restricts to the
+// states with that many set bits (down spins): the others are written as 0 without being evaluated.
 __global__ void __launch_bounds__(ED_THREADS) k_heis_matvec(const double *__restrict__ x, double *__restrict__ y,
                                                             unsigned dim, Bonds B, double qJ, double hJ,
-                                                            double *__restrict__ part, int popc) {
+                                                            GridSum R, int popc) {
     __shared__ unsigned sm[ED_MAX_BONDS];
     __shared__ double diag[ED_MAX_BONDS + 1];
     for (int i = threadIdx.x; i < B.nb; i += ED_THREADS) sm[i] = B.m[i];
@@ -113,14 +133,22 @@ __global__ void __launch_bounds__(ED_THREADS) k_heis_matvec(const double *__rest
             continue;
         }
         double off = 0.0;
-        int anti = 0;
-#pragma unroll 4
-        for (int b = 0; b < nlow; b++) {
-            const unsigned m = sm[b];
-            if (__popc(s & m) == 1) {
-                off += __ldg(x + (s ^ m));
-                anti++;
+        uint64_t lm = 0;                                 // this lane's antiparallel low bonds
+        for (int b = 0; b < nlow; b++) lm |= (uint64_t)(__popc(s & sm[b]) == 1) << b;
+        int anti = __popcll(lm);
+        while (lm) {
+            double v[2];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                v[j] = 0.0;
+                if (lm) {
+                    const int b = __ffsll((long long)lm) - 1;
+                    lm &= lm - 1;
+                    v[j] = __ldg(x + (s ^ sm[b]));
+                }
             }
+            off += v[0];                                 // in bond order (a spent lane adds zero)
+            off += v[1];
         }
         uint64_t hm = 0;                                 // antiparallel high bonds (same in all lanes)
         for (int b = nlow; b < nb; b++) hm |= (uint64_t)(__popc(s & sm[b]) == 1) << (b - nlow);
@@ -143,17 +171,17 @@ __global__ void __launch_bounds__(ED_THREADS) k_heis_matvec(const double *__rest
         y[s] = val;
         dot = fma(xs, val, dot);
     }
-    if (part) block_store(dot, part);
+    if (R.part) grid_sum(dot, R.part, R.ticket, [&](double t) { *R.out = t; });
 }
 
 // y[s] = scale * sum_e chi[e] x[pi_e(s)] over m group elements, pi_e(s) = OR_c tab[e][c][nibble c
-// of s] (bit i of pi_e(s) = bit perm_e[i] of s).  part (may be null) receives the block
-// partials of y.y.  popc >= 0: states whose popcount differs are set to 0 (the permutations
+// of s] (bit i of pi_e(s) = bit perm_e[i] of s).  R.part (may be null) takes the grid sum of y.y,
+// its root to *R.out.  popc >= 0: states whose popcount differs are set to 0 (the permutations
 // keep the popcount, so the sum for a state in the sector reads only states in it).
 __global__ void __launch_bounds__(ED_THREADS) k_perm_sum(const double *__restrict__ x, double *__restrict__ y,
                                                          unsigned dim, int m, const unsigned *__restrict__ tab,
-                                                         const double *__restrict__ chi, double scale,
-                                                         double *__restrict__ part, int popc) {
+                                                         const double *__restrict__ chi, double scale, GridSum R,
+                                                         int popc) {
     extern __shared__ __align__(16) unsigned char ed_smem[];
     double *s_chi = (double *)ed_smem;
     unsigned *s_tab = (unsigned *)(s_chi + m);
@@ -181,7 +209,7 @@ __global__ void __launch_bounds__(ED_THREADS) k_perm_sum(const double *__restric
         y[s] = v;
         nrm = fma(v, v, nrm);
     }
-    if (part) block_store(nrm, part);
+    if (R.part) grid_sum(nrm, R.part, R.ticket, [&](double t) { *R.out = sqrt(t); });
 }
 
 // out bit i of A x = parity(rows[i] & x): one GF(2) matrix of 64 rows.
@@ -215,15 +243,12 @@ __global__ void __launch_bounds__(ED_THREADS) k_lz_seed(double *__restrict__ v, 
     }
 }
 
-// w -= alpha v (+ beta_k v_prev for k > 0); alpha = sum of the matvec partials, stored in
-// al[k] by block 0 (src/mps/lanczos.c:903-912).
+// w -= alpha_k v (+ beta_k v_prev for k > 0), alpha and beta from the grid sums of the matvec and the
+// projector (src/mps/lanczos.c:903-912).
 __global__ void __launch_bounds__(ED_THREADS) k_lz_orth(double *__restrict__ w, const double *__restrict__ v,
-                                                        const double *__restrict__ vp, unsigned dim,
-                                                        const double *__restrict__ part, int np, double *al,
+                                                        const double *__restrict__ vp, unsigned dim, const double *al,
                                                         const double *be, int k) {
-    const double a = block_total(part, np);
-    if (blockIdx.x == 0 && threadIdx.x == 0) al[k] = a;
-    const double b = k > 0 ? be[k] : 0.0;
+    const double a = al[k], b = k > 0 ? be[k] : 0.0;
     const unsigned stride = gridDim.x * ED_THREADS;
     for (unsigned s = blockIdx.x * ED_THREADS + threadIdx.x; s < dim; s += stride) {
         double t = fma(-a, v[s], w[s]);
@@ -232,15 +257,21 @@ __global__ void __launch_bounds__(ED_THREADS) k_lz_orth(double *__restrict__ w, 
     }
 }
 
-// beta = sqrt(sum of the projector partials), stored in be[k+1] by block 0; unless beta is
-// below the breakdown bound, w *= 1/beta (src/mps/lanczos.c:945-947) and acc += z w.
-__global__ void __launch_bounds__(ED_THREADS) k_lz_scale(double *__restrict__ w, unsigned dim,
-                                                         const double *__restrict__ part, int np, double *be,
+// 1 / x by one thread of the block, for all of them (a division is seven FP64 instructions).
+__device__ __forceinline__ double block_reciprocal(double x) {
+    __shared__ double inv;
+    if (threadIdx.x == 0) inv = 1.0 / x;
+    __syncthreads();
+    return inv;
+}
+
+// Unless beta = be[k + 1] is below the breakdown bound, w *= 1/beta (src/mps/lanczos.c:945-947) and
+// acc += z w.
+__global__ void __launch_bounds__(ED_THREADS) k_lz_scale(double *__restrict__ w, unsigned dim, const double *be,
                                                          int k, double *__restrict__ acc, double z) {
-    const double b = sqrt(block_total(part, np));
-    if (blockIdx.x == 0 && threadIdx.x == 0) be[k + 1] = b;
+    const double b = be[k + 1];
     if (!(b >= ED_BETA_MIN)) return;
-    const double inv = 1.0 / b;
+    const double inv = block_reciprocal(b);
     const unsigned stride = gridDim.x * ED_THREADS;
     for (unsigned s = blockIdx.x * ED_THREADS + threadIdx.x; s < dim; s += stride) {
         const double t = w[s] * inv;
@@ -249,12 +280,10 @@ __global__ void __launch_bounds__(ED_THREADS) k_lz_scale(double *__restrict__ w,
     }
 }
 
-// n = sqrt(sum of partials) -> *nout; v /= n when n > 0 (src/mps/lanczos.c:884); acc = z v.
-__global__ void __launch_bounds__(ED_THREADS) k_lz_normalise(double *__restrict__ v, unsigned dim,
-                                                             const double *__restrict__ part, int np,
-                                                             double *nout, double *__restrict__ acc, double z) {
-    const double n = sqrt(block_total(part, np));
-    if (blockIdx.x == 0 && threadIdx.x == 0) *nout = n;
+// v /= n when n > 0 (src/mps/lanczos.c:884), n = *nout of the projector's grid sum; acc = z v.
+__global__ void __launch_bounds__(ED_THREADS) k_lz_normalise(double *__restrict__ v, unsigned dim, const double *nout,
+                                                             double *__restrict__ acc, double z) {
+    const double n = *nout;
     if (!(n > 0.0)) return;
     const unsigned stride = gridDim.x * ED_THREADS;
     for (unsigned s = blockIdx.x * ED_THREADS + threadIdx.x; s < dim; s += stride) {
@@ -264,21 +293,18 @@ __global__ void __launch_bounds__(ED_THREADS) k_lz_normalise(double *__restrict_
     }
 }
 
-// Block partials of x.x.
-__global__ void __launch_bounds__(ED_THREADS) k_sumsq(const double *__restrict__ x, unsigned dim,
-                                                      double *__restrict__ part) {
+// *R.out = ||x||.
+__global__ void __launch_bounds__(ED_THREADS) k_sumsq(const double *__restrict__ x, unsigned dim, GridSum R) {
     double t = 0.0;
     const unsigned stride = gridDim.x * ED_THREADS;
     for (unsigned s = blockIdx.x * ED_THREADS + threadIdx.x; s < dim; s += stride) t = fma(x[s], x[s], t);
-    block_store(t, part);
+    grid_sum(t, R.part, R.ticket, [&](double q) { *R.out = sqrt(q); });
 }
 
-// x *= 1 / ||x|| when ||x|| > 0 (src/mps/lanczos.c:1104-1105).
-__global__ void __launch_bounds__(ED_THREADS) k_unit(double *__restrict__ x, unsigned dim,
-                                                     const double *__restrict__ part, int np) {
-    const double n = sqrt(block_total(part, np));
-    if (!(n > 0.0)) return;
-    const double inv = 1.0 / n;
+// x *= 1 / n when n = ||x|| > 0 (src/mps/lanczos.c:1104-1105).
+__global__ void __launch_bounds__(ED_THREADS) k_unit(double *__restrict__ x, unsigned dim, const double *n) {
+    if (!(*n > 0.0)) return;
+    const double inv = block_reciprocal(*n);
     const unsigned stride = gridDim.x * ED_THREADS;
     for (unsigned s = blockIdx.x * ED_THREADS + threadIdx.x; s < dim; s += stride) x[s] *= inv;
 }
@@ -553,7 +579,7 @@ int ed_grid(unsigned dim) {
 }
 
 bool launch_perm_pass(const ProjPlan &P, int pass, const double *x, double *y, unsigned dim, double scale,
-                      double *part, cudaStream_t st, int popc = -1) {
+                      const GridSum &R, cudaStream_t st, int popc = -1) {
     static bool attr = false;
     if (!attr) {
         if (!NQS_CUDA(cudaFuncSetAttribute(k_perm_sum, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -567,18 +593,18 @@ bool launch_perm_pass(const ProjPlan &P, int pass, const double *x, double *y, u
     const size_t smem = (size_t)m * (ED_TAB * sizeof(unsigned) + sizeof(double));
     NQS_LAUNCH("ed_project_pass");
     k_perm_sum<<<ed_grid(dim), ED_THREADS, smem, st>>>(x, y, dim, m, P.tab.p + (size_t)off * ED_TAB,
-                                                       P.chi.p + off, scale, part, popc);
+                                                       P.chi.p + off, scale, R, popc);
     return NQS_CUDA(cudaGetLastError());
 }
 
 // Projects *a in place (using *t as scratch; the pointers may be swapped so that the
-// result is in *a).  part (may be null) receives the partials of the result's norm.
-bool project(const ProjPlan &P, double *&a, double *&t, unsigned dim, double *part, cudaStream_t st,
+// result is in *a).  R (R.part may be null) receives the result's norm.
+bool project(const ProjPlan &P, double *&a, double *&t, unsigned dim, const GridSum &R, cudaStream_t st,
              int popc = -1) {
     const double invG = 1.0 / (double)P.G;
     for (int k = 0; k < P.passes; k++) {
         const bool last = k + 1 == P.passes;
-        if (!launch_perm_pass(P, k, a, t, dim, last ? invG : 1.0, last ? part : nullptr, st, popc)) return false;
+        if (!launch_perm_pass(P, k, a, t, dim, last ? invG : 1.0, last ? R : GridSum{}, st, popc)) return false;
         std::swap(a, t);
     }
     return true;
@@ -718,7 +744,13 @@ struct EdVecs {
     DevBuf<double> v[4];
     DevBuf<double> acc;
     DevBuf<double> part, al, be, nrm;
+    DevBuf<unsigned> ticket;
 };
+
+// States up to which a run keeps its vectors for the next one (8 MB each; allocating and freeing them
+// is half a millisecond) and enqueues an iteration ahead of the host's convergence test (the one
+// too many at the end is below 0.1 ms there, the host's bisection up to 40 us an iteration).
+constexpr unsigned ED_SMALL_DIM = 1u << 20;
 
 std::vector<double> &last_alpha() {
     static std::vector<double> a;
@@ -762,13 +794,24 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
     if ((long)max_iters > (long)dim) max_iters = (int)dim;
     const int grid = ed_grid(dim);
     const size_t need = dim;
-    EdVecs E;
+    static EdVecs kept;
+    EdVecs own;
+    EdVecs &E = dim <= ED_SMALL_DIM ? kept : own;
     for (auto &b : E.v)
         if (!b.ensure(need)) return -1;
     if ((out_vec && !E.acc.ensure(need)) || !E.part.ensure(grid) || !E.al.ensure(max_iters + 1) ||
-        !E.be.ensure(max_iters + 2) || !E.nrm.ensure(1))
+        !E.be.ensure(max_iters + 2) || !E.nrm.ensure(1) || !E.ticket.ensure(1))
         return -1;
-    if (!NQS_CUDA(cudaMemsetAsync(E.be.p, 0, sizeof(double) * (max_iters + 2), st))) return -1;
+    if (!NQS_CUDA(cudaMemsetAsync(E.be.p, 0, sizeof(double) * (max_iters + 2), st)) ||
+        !NQS_CUDA(cudaMemsetAsync(E.ticket.p, 0, sizeof(unsigned), st)))
+        return -1;
+    auto sum_to = [&](double *out) {
+        GridSum R;
+        R.part = E.part.p;
+        R.ticket = E.ticket.p;
+        R.out = out;
+        return R;
+    };
     const double qJ = 0.25 * J, hJ = 0.5 * J;
     double *vc = E.v[0].p, *vp = E.v[1].p, *w = E.v[2].p, *t = E.v[3].p;
 
@@ -776,17 +819,17 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
     // leaves nothing, src/mps/lanczos.c:874-884); acc = z0 v0 on the replay
     int alt_used = 0;
     auto make_seed = [&](int alt, double *acc, double z0, double *norm_out) -> bool {
-        if (!launch_seed(vc, dim, alt, st, alt ? 0 : seed_state) || !project(*P, vc, t, dim, E.part.p, st, popc))
+        if (!launch_seed(vc, dim, alt, st, alt ? 0 : seed_state) || !project(*P, vc, t, dim, sum_to(E.nrm.p), st, popc))
             return false;
         if (seed_state && !alt) {
             // the caller-built seed: normalised once before the Lanczos projects it again
             NQS_LAUNCH("ed_normalise");
-            k_lz_normalise<<<grid, ED_THREADS, 0, st>>>(vc, dim, E.part.p, grid, E.nrm.p, nullptr, 0.0);
-            if (!NQS_CUDA(cudaGetLastError()) || !project(*P, vc, t, dim, E.part.p, st, popc)) return false;
+            k_lz_normalise<<<grid, ED_THREADS, 0, st>>>(vc, dim, E.nrm.p, nullptr, 0.0);
+            if (!NQS_CUDA(cudaGetLastError()) || !project(*P, vc, t, dim, sum_to(E.nrm.p), st, popc)) return false;
         }
         {
             NQS_LAUNCH("ed_normalise");
-            k_lz_normalise<<<grid, ED_THREADS, 0, st>>>(vc, dim, E.part.p, grid, E.nrm.p, acc, z0);
+            k_lz_normalise<<<grid, ED_THREADS, 0, st>>>(vc, dim, E.nrm.p, acc, z0);
         }
         if (!NQS_CUDA(cudaGetLastError())) return false;
         return NQS_CUDA(cudaMemcpyAsync(norm_out, E.nrm.p, sizeof(double), cudaMemcpyDeviceToHost, st)) &&
@@ -795,16 +838,16 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
     auto step = [&](int k, bool with_scale, double *acc, double z) -> bool {
         {
             NQS_LAUNCH("ed_matvec");
-            k_heis_matvec<<<grid, ED_THREADS, 0, st>>>(vc, w, dim, B, qJ, hJ, E.part.p, popc);
+            k_heis_matvec<<<grid, ED_THREADS, 0, st>>>(vc, w, dim, B, qJ, hJ, sum_to(E.al.p + k), popc);
         }
         {
             NQS_LAUNCH("ed_orth");
-            k_lz_orth<<<grid, ED_THREADS, 0, st>>>(w, vc, vp, dim, E.part.p, grid, E.al.p, E.be.p, k);
+            k_lz_orth<<<grid, ED_THREADS, 0, st>>>(w, vc, vp, dim, E.al.p, E.be.p, k);
         }
-        if (!NQS_CUDA(cudaGetLastError()) || !project(*P, w, t, dim, E.part.p, st, popc)) return false;
+        if (!NQS_CUDA(cudaGetLastError()) || !project(*P, w, t, dim, sum_to(E.be.p + k + 1), st, popc)) return false;
         if (with_scale) {
             NQS_LAUNCH("ed_scale");
-            k_lz_scale<<<grid, ED_THREADS, 0, st>>>(w, dim, E.part.p, grid, E.be.p, k, acc, z);
+            k_lz_scale<<<grid, ED_THREADS, 0, st>>>(w, dim, E.be.p, k, acc, z);
         }
         return NQS_CUDA(cudaGetLastError());
     };
@@ -824,13 +867,34 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
     std::vector<double> al(max_iters + 1, 0.0), be(max_iters + 2, 0.0);
     LeanOut o;
     int K = 0;
+    // alpha_k, beta_{k+1} of iteration k in slot k % 2 of a pinned pair, behind an event
+    struct Readback {
+        double *ab = nullptr;
+        cudaEvent_t done[2] = {};
+        bool ready() {
+            return ab || (NQS_CUDA(cudaMallocHost(&ab, 4 * sizeof(double))) &&
+                          NQS_CUDA(cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming)) &&
+                          NQS_CUDA(cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming)));
+        }
+    };
+    static Readback rb;
+    if (!rb.ready()) return -1;
+    auto iterate = [&](int k) -> bool {
+        double *ab = rb.ab + 2 * (k & 1);
+        return step(k, true, nullptr, 0.0) &&
+               NQS_CUDA(cudaMemcpyAsync(&ab[0], E.al.p + k, sizeof(double), cudaMemcpyDeviceToHost, st)) &&
+               NQS_CUDA(cudaMemcpyAsync(&ab[1], E.be.p + k + 1, sizeof(double), cudaMemcpyDeviceToHost, st)) &&
+               NQS_CUDA(cudaEventRecord(rb.done[k & 1], st));
+    };
+    const bool ahead = dim <= ED_SMALL_DIM;
+    if (!iterate(0)) return -1;
     for (int k = 0; k < max_iters; k++) {
-        if (!step(k, true, nullptr, 0.0)) return -1;
-        double ab[2];
-        if (!NQS_CUDA(cudaMemcpyAsync(&ab[0], E.al.p + k, sizeof(double), cudaMemcpyDeviceToHost, st)) ||
-            !NQS_CUDA(cudaMemcpyAsync(&ab[1], E.be.p + k + 1, sizeof(double), cudaMemcpyDeviceToHost, st)) ||
-            !NQS_CUDA(cudaStreamSynchronize(st)))
-            return -1;
+        if (ahead && k + 1 < max_iters) {
+            rotate();
+            if (!iterate(k + 1)) return -1;
+        }
+        if (!NQS_CUDA(cudaEventSynchronize(rb.done[k & 1]))) return -1;
+        const double *ab = rb.ab + 2 * (k & 1);
         al[k] = ab[0];
         be[k + 1] = ab[1];
         K = k + 1;
@@ -841,7 +905,10 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
             o.converged = 1;
             break;
         }
-        rotate();
+        if (!ahead && k + 1 < max_iters) {
+            rotate();
+            if (!iterate(k + 1)) return -1;
+        }
     }
     o.iters = K;
     last_alpha().assign(al.begin(), al.begin() + K);
@@ -875,8 +942,8 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
     }
     {
         NQS_LAUNCH("ed_normalise");
-        k_sumsq<<<grid, ED_THREADS, 0, st>>>(E.acc.p, dim, E.part.p);
-        k_unit<<<grid, ED_THREADS, 0, st>>>(E.acc.p, dim, E.part.p, grid);
+        k_sumsq<<<grid, ED_THREADS, 0, st>>>(E.acc.p, dim, sum_to(E.nrm.p));
+        k_unit<<<grid, ED_THREADS, 0, st>>>(E.acc.p, dim, E.nrm.p);
     }
     if (!NQS_CUDA(cudaGetLastError()) ||
         !NQS_CUDA(cudaMemcpyAsync(out_vec, E.acc.p, sizeof(double) * (size_t)dim, cudaMemcpyDeviceToHost, st)) ||
@@ -944,7 +1011,7 @@ int nqs_gpu_kagome_heis_matvec(int Lx, int Ly, double J, int pbc, const double *
     {
         NQS_LAUNCH("ed_matvec");
         k_heis_matvec<<<ed_grid(dim), ED_THREADS, 0, ctx().stream>>>(d_in, d_out, dim, B, 0.25 * J, 0.5 * J,
-                                                                     nullptr, -1);
+                                                                     GridSum{}, -1);
     }
     return NQS_CUDA(cudaGetLastError()) ? 0 : -1;
 }
@@ -969,7 +1036,7 @@ int nqs_gpu_sector_project(int N, int G, const int *perm, const double *chars, c
         const bool last = k + 1 == P->passes;
         double *dst = last ? d_out : tmp[k % 2].p;
         if (dst == src) dst = tmp[0].p;              // a single pass in place: copied back below
-        if (!launch_perm_pass(*P, k, src, dst, dim, last ? invG : 1.0, nullptr, st)) return -1;
+        if (!launch_perm_pass(*P, k, src, dst, dim, last ? invG : 1.0, GridSum{}, st)) return -1;
         src = dst;
     }
     if (src != d_out &&
@@ -1026,7 +1093,7 @@ void nqs_kagome_p6m_project_inplace(double *psi, int N, int G, const int *perm, 
     if (!a.ensure(dim) || !t.ensure(dim)) return;
     double *pa = a.p, *pt = t.p;
     if (!NQS_CUDA(cudaMemcpyAsync(pa, psi, sizeof(double) * dim, cudaMemcpyHostToDevice, st)) ||
-        !project(*P, pa, pt, dim, nullptr, st))
+        !project(*P, pa, pt, dim, GridSum{}, st))
         return;
     if (NQS_CUDA(cudaMemcpyAsync(psi, pa, sizeof(double) * dim, cudaMemcpyDeviceToHost, st)))
         NQS_CUDA(cudaStreamSynchronize(st));
