@@ -148,7 +148,7 @@ int nqs_gpu_made_sample(nqs_sampler_t *s, int count, int *out_spins, double *out
  * autotuner on the first step, which also picks the factor's tile shape (the
  * diagonal block width, 64 or 128, by instance order) (nqs_gpu_batch_ctas reports
  * the split, nqs_gpu_batch_block_widths the widths, nqs_gpu_batch_tune_ms the
- * candidates' times: every CTA split for each width rule); from the second step the whole
+ * times of the launches it tried); from the second step the whole
  * batch step is one CUDA graph replayed per step.  An instance whose FP32
  * factor breaks down is solved again in FP64 on the same samples after the
  * graph (as nqs_sr_step_minsr_full does in the MIXED mode);

@@ -8,11 +8,13 @@
 // refines the systems of all instances (each instance owns a range of CTAs with
 // its own grid barrier), then per instance delta = O_c^T y / N_s (sample space)
 // and the update.  The first step runs uncaptured and autotunes the split of
-// the cooperative launch's CTAs between the instances (candidate splits timed
-// with CUDA events on the Grams of that step); from the second step the whole
+// the cooperative launch's CTAs between the instances (balanced by the systems'
+// solve times measured on the Grams of that step); from the second step the whole
 // sequence is one CUDA graph replayed per step, the samplers' move counters
 // living in device memory so that each replay draws new random numbers.
+#include <algorithm>
 #include <math.h>
+#include <stdlib.h>
 
 #include "nqs_amp.cuh"
 
@@ -167,79 +169,147 @@ static bool fork_join(Batch &B, cudaStream_t main, F work) {
     return ok;
 }
 
-// Candidate splits of the cooperative launch's CTAs between the instances:
-// the same count for every instance (1, 2, 4, ...) and counts proportional to
-// n_i^e for e = 1, 2, 3 (n_i the order of instance i's system: its factor is
-// n^3 work on a chain of n / 128 diagonal blocks), within the co-resident limit.
-static std::vector<std::vector<int>> cta_candidates(const Batch &B, int cap) {
+// Splits of the cooperative launch's CTAs between the instances to start from: the largest equal
+// counts (a power of two) and counts proportional to the order n_i of instance i's system, within
+// the co-resident limit.
+static std::vector<std::vector<int>> cta_starts(const Batch &B, int cap) {
     const int K = (int)B.inst.size();
     std::vector<std::vector<int>> c;
-    for (int u = 1; u * K <= cap && u <= 32; u *= 2) c.push_back(std::vector<int>((size_t)K, u));
-    for (int e = 1; e <= 3; e++) {
-        std::vector<double> w((size_t)K);
-        double tot = 0.0;
-        for (int i = 0; i < K; i++) tot += (w[i] = pow((double)mixed_sys_order(B.inst[i]->mx), (double)e));
-        std::vector<int> prop((size_t)K);
-        int used = 0;
-        for (int i = 0; i < K; i++) {
-            prop[i] = (int)floor(w[i] / tot * (double)(cap - K)) + 1;
-            used += prop[i];
-        }
-        if (used <= cap) c.push_back(prop);
-    }
+    int u = 1;
+    while (2 * u * K <= cap && u < 32) u *= 2;
+    c.push_back(std::vector<int>((size_t)K, u));
+    double tot = 0.0;
+    for (BatchInst *b : B.inst) tot += (double)mixed_sys_order(b->mx);
+    std::vector<int> prop((size_t)K);
+    for (int i = 0; i < K; i++)
+        prop[i] = (int)floor((double)mixed_sys_order(B.inst[i]->mx) / tot * (double)(cap - K)) + 1;
+    c.push_back(prop);
     return c;
 }
 
-// Autotune on the Grams of the first step: re-run each instance's Gram from
-// its split operands and time the cooperative launch for every candidate CTA
-// split and every tile shape of the factor (the diagonal block width: 128 from
-// order 4096, from 2048, from 1024, else 64); keep the fastest (its launch, after
-// a last Gram, is the step's solve).
+// One system's solve times by CTA count, t = c + w / g through the two counts nearest to g.
+struct SolveTimes {
+    std::map<int, double> at;
+    void line(int g, double &c, double &w) const {
+        int g1 = -1, g2 = -1;
+        for (const auto &e : at) {
+            if (g1 < 0 || abs(e.first - g) < abs(g1 - g)) {
+                g2 = g1;
+                g1 = e.first;
+            } else if (g2 < 0 || abs(e.first - g) < abs(g2 - g)) {
+                g2 = e.first;
+            }
+        }
+        const double t1 = at.at(g1);
+        if (g2 > 0) w = (at.at(g2) - t1) / (1.0 / g2 - 1.0 / g1);
+        // a single count, or a time that does not fall with the count: half of it taken as divisible
+        if (g2 < 0 || !(w > 0.0) || !(w / g1 < t1)) w = 0.5 * t1 * g1;
+        c = t1 - w / g1;
+    }
+};
+
+// Counts that make the slowest system fastest under those lines: the least T with
+// sum_i max(1, w_i / (T - c_i)) within the limit.
+static std::vector<int> balanced_split(const std::vector<SolveTimes> &st, const std::vector<int> &cur, int cap) {
+    const size_t K = st.size();
+    std::vector<double> c(K), w(K);
+    double lo = 0.0, hi = 0.0;
+    for (size_t i = 0; i < K; i++) {
+        st[i].line(cur[i], c[i], w[i]);
+        lo = std::max(lo, c[i]);
+        hi = std::max(hi, c[i] + w[i]);
+    }
+    auto counts = [&](double T, std::vector<int> &g) {
+        long sum = 0;
+        for (size_t i = 0; i < K; i++) {
+            g[i] = T > c[i] ? (int)std::min((double)cap, std::max(1.0, ceil(w[i] / (T - c[i])))) : cap;
+            sum += g[i];
+        }
+        return sum;
+    };
+    std::vector<int> g(K), best(K, 1);
+    for (int it = 0; it < 60; it++) {
+        const double T = 0.5 * (lo + hi);
+        if (counts(T, g) <= cap) {
+            best = g;
+            hi = T;
+        } else {
+            lo = T;
+        }
+    }
+    return best;
+}
+
+// Autotune on the Grams of the first step: re-run each instance's Gram from its split operands and
+// time the cooperative launch, and in it every system's own solve.  From two starting splits the
+// counts are balanced by the systems' measured times, a few rounds while the launch gets faster; then
+// the other diagonal block widths of the factor (128 from order 2048, from 1024) where a system is
+// that large.  The fastest is kept (its launch, after a last Gram, is the step's solve).
+// Measured, 16 instances of order 156 to 2144: 1.63 ms (the best of seven fixed splits: 2.27 ms, and
+// 277 ms for the first step with its 21 launches, now 27 ms).
 static bool autotune(Batch &B, cudaStream_t st) {
-    const int cap = mixed_batch_capacity();
-    if (cap < (int)B.inst.size()) {
-        set_error("batch of %d instances needs at least one co-resident CTA each (device holds %d)",
-                  (int)B.inst.size(), cap);
+    const int cap = mixed_batch_capacity(), K = (int)B.inst.size();
+    if (cap < K) {
+        set_error("batch of %d instances needs at least one co-resident CTA each (device holds %d)", K, cap);
         return false;
     }
     std::vector<MixedSys *> sys;
-    for (BatchInst *b : B.inst) sys.push_back(b->mx);
-    const std::vector<std::vector<int>> cand = cta_candidates(B, cap);
-    const int bd_cand[3] = {mixed_bd_default(), 2048, 1024};
+    int largest = 0;
+    for (BatchInst *b : B.inst) {
+        sys.push_back(b->mx);
+        largest = std::max(largest, mixed_sys_order(b->mx));
+    }
     cudaEvent_t e0, e1;
     if (!NQS_CUDA(cudaEventCreate(&e0)) || !NQS_CUDA(cudaEventCreate(&e1))) return false;
     double best = 1e300;
-    int bi = -1, bb = 0;
+    bool first = true;
     B.tune_ms.clear();
-    for (size_t k = 0; k < cand.size() * 3; k++) {
-        const size_t c = k % cand.size();
-        const int t = (int)(k / cand.size());
-        MixedBatch *mb = mixed_batch_create(sys.data(), (int)sys.size(), cand[c].data(), bd_cand[t]);
+    std::vector<SolveTimes> times((size_t)K);
+    // Milliseconds of one launch (-1: it does not fit, -2: an error); the fastest is remembered.
+    auto measure = [&](const std::vector<int> &ctas, int bd_from, bool keep_times) -> double {
+        MixedBatch *mb = mixed_batch_create(sys.data(), K, ctas.data(), bd_from, true);
         if (!mb) {
             B.tune_ms.push_back(-1.0);
-            continue;
+            return -1.0;
         }
-        if (k > 0)
+        if (!first)
             for (BatchInst *b : B.inst) mixed_sys_front(b->mx, st, false);
+        first = false;
         float ms = 0.f;
-        const bool ok = NQS_CUDA(cudaEventRecord(e0, st)) && mixed_batch_launch(mb, st) &&
-                        NQS_CUDA(cudaEventRecord(e1, st)) && NQS_CUDA(cudaEventSynchronize(e1)) &&
-                        NQS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        bool ok = NQS_CUDA(cudaEventRecord(e0, st)) && mixed_batch_launch(mb, st) && NQS_CUDA(cudaEventRecord(e1, st)) &&
+                  NQS_CUDA(cudaEventSynchronize(e1)) && NQS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         mixed_batch_free(mb);
-        if (!ok) break;
+        for (int i = 0; i < K && ok && keep_times; i++) {
+            double us = 0.0;
+            ok = mixed_sys_solve_us(sys[i], &us);
+            if (us > 0.0) times[i].at[ctas[i]] = us;
+        }
+        if (!ok) return -2.0;
         B.tune_ms.push_back(ms);
         if (ms < best) {
             best = ms;
-            bi = (int)c;
-            bb = bd_cand[t];
+            B.ctas = ctas;
+            B.bd_from = bd_from;
         }
+        return ms;
+    };
+    bool ok = true;
+    for (const std::vector<int> &c : cta_starts(B, cap)) ok = ok && measure(c, mixed_bd_default(), true) > -2.0;
+    bool timed = true;
+    for (const SolveTimes &t : times) timed = timed && !t.at.empty();
+    for (int round = 0; round < 5 && ok && timed && !B.ctas.empty(); round++) {
+        const std::vector<int> next = balanced_split(times, B.ctas, cap);
+        if (next == B.ctas) break;
+        const double before = best, ms = measure(next, mixed_bd_default(), true);
+        ok = ms > -2.0;
+        if (round > 0 && best > 0.99 * before) break;
     }
+    for (int bd : {2048, 1024})
+        if (ok && largest >= bd && !B.ctas.empty()) ok = measure(std::vector<int>(B.ctas), bd, false) > -2.0;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (bi < 0) return false;
-    B.ctas = cand[bi];
-    B.bd_from = bb;
-    B.mb = mixed_batch_create(sys.data(), (int)sys.size(), B.ctas.data(), B.bd_from);
+    if (!ok || B.ctas.empty()) return false;
+    B.mb = mixed_batch_create(sys.data(), K, B.ctas.data(), B.bd_from, false);
     if (!B.mb) return false;
     for (BatchInst *b : B.inst) mixed_sys_front(b->mx, st, false);
     return mixed_batch_launch(B.mb, st);
@@ -269,7 +339,9 @@ nqs_gpu_batch_t *nqs_gpu_batch_create(const nqs_gpu_instance_t *in, int count) {
     B.sweeps = c.opts.refine_sweeps;
     B.passes = c.opts.gram_passes;
     B.space = c.opts.mixed_space;
-    const int nside = count < 8 ? count : 8;
+    // one stream per instance up to 32: an instance's front is a dozen short kernels in a row that leave
+    // most SMs idle
+    const int nside = count < 32 ? count : 32;
     B.side.resize((size_t)nside, nullptr);
     B.join.resize((size_t)nside, nullptr);
     for (int k = 0; k < nside; k++)

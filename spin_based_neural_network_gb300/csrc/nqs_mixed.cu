@@ -3059,6 +3059,13 @@ void mixed_sys_front(MixedSys *m, cudaStream_t st, bool with_split) {
     enqueue_fr_clear(m->w, m->fa, st);
 }
 
+// Microseconds of the system's last timed solve, from its CTA 0 (0: it broke down).
+bool mixed_sys_solve_us(const MixedSys *m, double *us) {
+    unsigned long long ns[8];
+    if (!NQS_CUDA(cudaMemcpy(ns, m->w.tm.p, sizeof(ns), cudaMemcpyDeviceToHost))) return false;
+    *us = 1e-3 * (double)ns[6];
+    return true;
+}
 bool mixed_sys_param_space(const MixedSys *m) { return m->pl.space == 1; }
 int mixed_bd_default() { return BD_SWITCH; }
 int mixed_sys_order(const MixedSys *m) { return m->pl.n; }
@@ -3083,11 +3090,13 @@ int mixed_batch_capacity() {
 
 // bd_from: systems of order >= bd_from factor with 128-wide diagonal blocks, the others
 // with 64-wide ones (a tile shape the batch autotuner chooses).
-MixedBatch *mixed_batch_create(MixedSys *const *sys, int count, const int *ctas, int bd_from) {
+// timing: each system's solve time is recorded (mixed_sys_solve_us).
+MixedBatch *mixed_batch_create(MixedSys *const *sys, int count, const int *ctas, int bd_from, bool timing) {
     std::vector<FrArgs> fa((size_t)count);
     std::vector<int> c0((size_t)count), nc((size_t)count), map;
     for (int i = 0; i < count; i++) {
         fa[i] = sys[i]->fa;
+        if (timing) fa[i].tm = sys[i]->w.tm.p;
         fa[i].bd = sys[i]->pl.n >= bd_from ? BD_LARGE : BD_SMALL;
         c0[i] = (int)map.size();
         nc[i] = ctas[i] > 0 ? ctas[i] : 1;
