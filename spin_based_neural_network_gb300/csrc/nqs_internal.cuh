@@ -248,11 +248,13 @@ constexpr double MIXED_RESID_MAX = 1e-6;
 // after_launch, when given, is called once the solve is enqueued and before the host waits for
 // it, with the solve's status word, error word and residual norms (device pointers) and
 // whether it solves in parameter space, so that a caller can enqueue work that depends on
-// the solve without a host round trip.
+// the solve without a host round trip.  eps_ready, when given, is the event behind which eps is
+// written (the front of the solve does not read it).
 using MixedAfterLaunch = std::function<bool(const int *status, const int *err, const double *nrm, bool param_space)>;
 bool minsr_mixed_solve(double *O, const double *gm, const double *eps, int Ns, long P, double shift, int sweeps,
                        int passes, int space_opt, double *y, double *delta, bool *param_space, double *out_resid,
-                       int *out_fail, const MixedAfterLaunch &after_launch = nullptr);
+                       int *out_fail, const MixedAfterLaunch &after_launch = nullptr,
+                       cudaEvent_t eps_ready = nullptr);
 
 // theta -= lr delta and ||delta||^2 into scal[S_NORM2] on the library stream, with delta
 // taken as zero when the mixed solve broke down (a non-positive FP32 pivot in status[0], or

@@ -2462,9 +2462,11 @@ static void enqueue_fr_clear(MixedWs &w, const FrArgs &fa, cudaStream_t st) {
 
 static void enqueue_mixed(const MixedPlan &pl, double *O, const double *gm, const double *eps, int Ns, long P,
                           double shift, int sweeps, int passes, double *x, const CUtensorMap &mh,
-                          const CUtensorMap &ml, int *err, cudaStream_t st) {
+                          const CUtensorMap &ml, int *err, cudaStream_t st, cudaEvent_t eps_ready, bool captured) {
     MixedWs &w = g_mx;
     enqueue_front(w, pl, O, gm, Ns, P, shift, passes, mh, ml, err, st);
+    // (in a graph: a node that waits for the event's record before each replay)
+    if (eps_ready) NQS_CUDA(cudaStreamWaitEvent(st, eps_ready, captured ? cudaEventWaitExternal : 0));
     const FrArgs fa = make_frargs(w, pl, O, eps, Ns, P, shift, sweeps, x, err);
     enqueue_fr_clear(w, fa, st);
     cudaLaunchConfig_t lc = {};
@@ -2562,7 +2564,7 @@ static bool ensure_attrs() {
 // profiling runs the sequence uncaptured.
 struct MixedGraph {
     cudaGraphExec_t exec = nullptr;
-    const void *key[5] = {};
+    const void *key[6] = {};
     int Ns = 0, sweeps = -1, passes = -1, space = -1;
     long P = 0;
     double shift = 0.0;
@@ -2572,7 +2574,7 @@ static MixedGraph g_mgraph;
 
 bool minsr_mixed_solve(double *O, const double *gm, const double *eps, int Ns, long P, double shift, int sweeps,
                        int passes, int space_opt, double *y, double *delta, bool *param_space, double *out_resid,
-                       int *out_fail, const MixedAfterLaunch &after_launch) {
+                       int *out_fail, const MixedAfterLaunch &after_launch, cudaEvent_t eps_ready) {
     Context &c = ctx();
     cudaStream_t st = c.stream;
     MixedWs &w = g_mx;
@@ -2587,20 +2589,20 @@ bool minsr_mixed_solve(double *O, const double *gm, const double *eps, int Ns, l
     double *x = pl.space ? delta : y;
 
     if (c.profiling) {
-        enqueue_mixed(pl, O, gm, eps, Ns, P, shift, sweeps, passes, x, mh, ml, err.p, st);
+        enqueue_mixed(pl, O, gm, eps, Ns, P, shift, sweeps, passes, x, mh, ml, err.p, st, eps_ready, false);
     } else {
         MixedGraph &Gr = g_mgraph;
-        const void *key[5] = {O, gm, eps, x, w.hi.p};
+        const void *key[6] = {O, gm, eps, x, w.hi.p, eps_ready};
         bool same = Gr.exec && !moved && Gr.Ns == Ns && Gr.P == P && Gr.sweeps == sweeps &&
                     Gr.passes == passes && Gr.shift == shift && Gr.space == pl.space;
-        for (int i = 0; i < 5 && same; i++) same = Gr.key[i] == key[i];
+        for (int i = 0; i < 6 && same; i++) same = Gr.key[i] == key[i];
         if (!same) {
             if (Gr.exec) cudaGraphExecDestroy(Gr.exec);
             Gr.exec = nullptr;
             cudaGraph_t graph;
             const long l0 = c.launches;
             if (!NQS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal))) return false;
-            enqueue_mixed(pl, O, gm, eps, Ns, P, shift, sweeps, passes, x, mh, ml, err.p, st);
+            enqueue_mixed(pl, O, gm, eps, Ns, P, shift, sweeps, passes, x, mh, ml, err.p, st, eps_ready, true);
             if (!NQS_CUDA(cudaStreamEndCapture(st, &graph))) return false;
             Gr.kernels = c.launches - l0;
             c.launches = l0;
@@ -2610,7 +2612,7 @@ bool minsr_mixed_solve(double *O, const double *gm, const double *eps, int Ns, l
                 Gr.exec = nullptr;
                 return false;
             }
-            for (int i = 0; i < 5; i++) Gr.key[i] = key[i];
+            for (int i = 0; i < 6; i++) Gr.key[i] = key[i];
             Gr.Ns = Ns;
             Gr.P = P;
             Gr.sweeps = sweeps;
