@@ -50,3 +50,13 @@ def test_widths(nqs, kind, M):
 def test_peaked_states_and_weights_out_of_range(nqs, kind, scale):
     for exchange in (False, True):
         chains(nqs, kind, 4, 4, 24, scale, exchange, 7, 35, 11, 5)
+
+
+@pytest.mark.parametrize("kind", [O.OR_RBM, O.OR_CRBM])
+@pytest.mark.parametrize("M", [1, 5, 16])
+@pytest.mark.parametrize("scale", [0.02, 0.8, 2.5, 60.0])
+def test_two_proposals_a_round(nqs, kind, M, scale):
+    # nearly free chains (both proposals accepted), peaked ones, and weights out of range; an odd
+    # number of moves, records at every move and across the 32-move draws
+    chains(nqs, kind, 9, 1, M, scale, False, 6, 6 * 41, 1, 11)
+    chains(nqs, kind, 4, 4, M, scale, False, 3, 3 * 5, 31, 12)
