@@ -3,15 +3,15 @@
 //
 // 32-wide block columns, right-looking.  Step k:
 //   panel     the rows below the factored diagonal block, x L_kk^T = a, and the right-hand side,
-//             eight rows a warp with four lanes a row, spread over the CTAs so that each SM's
-//             FP64 pipe takes a share (a warp instruction takes 16 clocks of it however many
-//             lanes are active);
+//             two or eight rows a warp with 16 or four lanes a row, spread over the CTAs so that
+//             each SM's FP64 pipes take a share (a warp instruction takes 64 clocks of a quarter
+//             SM's pipe however many lanes are active);
 //   trailing  32 x 32 tiles of A -= P P^T (and of z -= P z_k, by the owners of the diagonal tiles)
 //             on CTAs 1 .. G-1, while CTA 0 updates the next diagonal block and factors it.
 // The step is bound by the FP64 pipes of all SMs while the trailing matrix is large and by the
 // chain panel -> next diagonal block -> two grid barriers below n ~ 1000 (an FP64 instruction takes
 // 64 clocks of a quarter SM's pipe and as long to return, so a chain of them is slow wherever it runs).
-// Measured at n = 1000 (4x4 Heisenberg, 1000 samples): 1.69 ms for factor and solve against 5.85 ms
+// Measured at n = 1000 (4x4 Heisenberg, 1000 samples): 1.23 ms for factor and solve against 5.85 ms
 // as 157 launches of one kernel per block and phase.
 #include <algorithm>
 
@@ -49,55 +49,100 @@ __device__ __forceinline__ void lower_tile(int t, int &bi, int &bj) {
     bj = t - r * (r + 1) / 2;
 }
 
-// Factor the kb x kb block in S (lower triangle; lane = row, in registers) by one warp; rinv gets
-// the reciprocal pivots.  Returns the first column whose pivot is not positive, or -1; the
-// columns before it are finished in S (the pivot test of src/nqs/nqs_optimizer.c:1029-1031).
-__device__ int factor32(double (*S)[CB + 1], int kb, double *rinv, double *col) {
-    const int lane = threadIdx.x & 31;
-    double d[CB];
+// Factor the kb x kb block in S (lower triangle; rows kb .. 31 the identity) by the block, in panels of
+// four columns: warp 0 (lane = row) runs the panel's pivots and their columns in registers, then all
+// warps take the panel off the columns after it, so that the long part of the FP64 work is on the four
+// pipes of the SM and warp 0 keeps the chain of pivots only (34 FP64 instructions a panel).  rinv gets
+// the reciprocal pivots; *fail the first column whose pivot is not positive, or -1; the columns
+// before it are finished in S (the pivot test of src/nqs/nqs_optimizer.c:1029-1031).
+// Measured: order 1000, factor and solve 1.23 ms, 1.69 ms with the whole block by one warp (28 us each)
+// and eight rows a warp in every panel.
+__device__ void factor32(double (*S)[CB + 1], int kb, double *rinv, int *fail) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int j0 = 0; j0 < CB; j0 += 4) {
+        if (warp == 0) {
+            double d[4];
+            int f = -1;
 #pragma unroll
-    for (int j = 0; j < CB; j++) d[j] = lane < kb && j <= lane ? S[lane][j] : (j == lane ? 1.0 : 0.0);
-    int fail = -1;
+            for (int b = 0; b < 4; b++) d[b] = lane >= j0 + b ? S[lane][j0 + b] : 0.0;
 #pragma unroll
-    for (int j = 0; j < CB; j++) {
-        double p = __shfl_sync(0xffffffffu, d[j], j);
-        if (fail < 0 && j < kb && !(p > 0.0)) fail = j;
-        if (fail >= 0) p = 1.0;                        // the sweep ends on a unit pivot
-        const double y = rsqrt(p), l = d[j] * y;
-        if (lane == j) rinv[j] = y;
-        if (fail < 0) d[j] = l;
-        double *c = col + (j & 1) * CB;
-        c[lane] = l;
-        __syncwarp();
+            for (int b = 0; b < 4; b++) {
+                double p = __shfl_sync(0xffffffffu, d[b], j0 + b);
+                if (f < 0 && j0 + b < kb && !(p > 0.0)) f = j0 + b;
+                if (f >= 0) p = 1.0;                        // the sweep ends on a unit pivot
+                const double y = rsqrt(p), l = d[b] * y;
+                if (lane == j0 + b) rinv[j0 + b] = y;
+                if (f < 0) d[b] = l;
 #pragma unroll
-        for (int k = j + 1; k < CB; k++) d[k] = fma(-l, c[k], d[k]);
+                for (int c = b + 1; c < 4; c++) d[c] = fma(-l, __shfl_sync(0xffffffffu, l, j0 + c), d[c]);
+            }
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+                if (lane >= j0 + b && (f < 0 || j0 + b < f)) S[lane][j0 + b] = d[b];
+            if (lane == 0) *fail = f;
+        }
+        __syncthreads();
+        if (*fail >= 0) return;                             // the same for the whole block
+        const int r0 = j0 + 4, i = tid >> 3;
+        if (4 * warp + 3 >= r0) {                           // warp w: rows 4 w .. 4 w + 3
+            double l[4];
+#pragma unroll
+            for (int b = 0; b < 4; b++) l[b] = S[i][j0 + b];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int c = (tid & 7) + 8 * q;
+                if (c >= r0 && c <= i) {
+                    double v = S[i][c];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) v = fma(-l[b], S[c][j0 + b], v);
+                    S[i][c] = v;
+                }
+            }
+        }
+        __syncthreads();
     }
-    __syncwarp();
-    const int keep = fail < 0 ? kb : fail;
-#pragma unroll
-    for (int j = 0; j < CB; j++)
-        if (j <= lane && j < keep && lane < kb) S[lane][j] = d[j];
-    return fail;
 }
 
-// x of one row from a (8 columns q + 4 i a lane, four lanes a row): x_j = a_j / L_jj, a -= x_j L_:j.
-__device__ __forceinline__ void row_solve(double (&s)[8], const double (*Ld)[CB + 1], const double *rinv, int kb,
+// x of one row from a (columns q + LR i a lane, LR lanes a row): x_j = a_j / L_jj, a -= x_j L_:j.
+template <int LR>
+__device__ __forceinline__ void row_solve(double (&s)[CB / LR], const double (*Ld)[CB + 1], const double *rinv, int kb,
                                           int lane) {
-    const int q = lane & 3;
+    const int q = lane % LR;
 #pragma unroll
     for (int j = 0; j < CB; j++) {
         if (j >= kb) break;
-        const int i = j >> 2;
-        const double x = __shfl_sync(0xffffffffu, s[i] * rinv[j], (lane & ~3) | (j & 3));
-        if (q == (j & 3)) s[i] = x;
+        const int i = j / LR;
+        const double x = __shfl_sync(0xffffffffu, s[i] * rinv[j], (lane & ~(LR - 1)) | (j % LR));
+        if (q == j % LR) s[i] = x;
 #pragma unroll
-        for (int k = i; k < 8; k++) s[k] = fma(-x, Ld[q + 4 * k][j], s[k]);   // zero at and above the diagonal
+        for (int k = i; k < CB / LR; k++) s[k] = fma(-x, Ld[q + LR * k][j], s[k]);   // zero at and above the diagonal
+    }
+}
+
+// The panel of the block at k0 (unit diagonal block Ld, reciprocal pivots rinv) and the right-hand
+// side: 32 / LR rows a warp, dealt to the CTAs first.
+template <int LR>
+__device__ __forceinline__ void panel_solve(double *T, double *z, int n, int k0, int kb, const double (*Ld)[CB + 1],
+                                            const double *rinv) {
+    constexpr int RW = 32 / LR, C = CB / LR;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k1 = k0 + kb, q = lane % LR;
+    const int nun = (n - k1 + RW - 1) / RW;                 // unit nun is the right-hand side
+    for (int u = blockIdx.x + gridDim.x * warp; u <= nun; u += gridDim.x * (CT / 32)) {
+        const int row = k1 + u * RW + lane / LR;
+        const bool ok = u < nun ? row < n : lane < LR;
+        double *p = u < nun ? T + (size_t)row * n + k0 : z + k0;
+        double s[C];
+#pragma unroll
+        for (int i = 0; i < C; i++) s[i] = ok && q + LR * i < kb ? __ldcg(p + q + LR * i) : 0.0;
+        row_solve<LR>(s, Ld, rinv, kb, lane);
+#pragma unroll
+        for (int i = 0; i < C; i++)
+            if (ok && q + LR * i < kb) p[q + LR * i] = s[i];
     }
 }
 
 __global__ void __launch_bounds__(CT, 1) k_chol64(Chol64Args a) {
     __shared__ Chol64Smem sm;
-    __shared__ double col[2 * CB];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bx = blockIdx.x, G = gridDim.x;
     const int n = a.n, nblk = (n + CB - 1) / CB;
     double *T = a.T;
@@ -105,11 +150,7 @@ __global__ void __launch_bounds__(CT, 1) k_chol64(Chol64Args a) {
     // CTA 0: the diagonal block at k0 from sm.A, factored and stored
     auto factor_store = [&](int k0) {
         const int kb = min(CB, n - k0);
-        if (warp == 0) {
-            const int f = factor32(sm.A, kb, sm.rinv, col);
-            if (lane == 0) sm.fail = f;
-        }
-        __syncthreads();
+        factor32(sm.A, kb, sm.rinv, &sm.fail);
         const int f = sm.fail, keep = f < 0 ? kb : f;
         for (int e = tid; e < CB * CB; e += CT) {
             const int r = e >> 5, c = e & 31;
@@ -121,7 +162,7 @@ __global__ void __launch_bounds__(CT, 1) k_chol64(Chol64Args a) {
     if (bx == 0) {
         for (int e = tid; e < CB * CB; e += CT) {
             const int r = e >> 5, c = e & 31;
-            sm.A[r][c] = r < n && c <= r ? T[(size_t)r * n + c] : 0.0;
+            sm.A[r][c] = r < n && c <= r ? T[(size_t)r * n + c] : (r == c ? 1.0 : 0.0);
         }
         __syncthreads();
         factor_store(0);
@@ -131,26 +172,18 @@ __global__ void __launch_bounds__(CT, 1) k_chol64(Chol64Args a) {
         const int k0 = k * CB, kb = min(CB, n - k0), k1 = k0 + kb, rest = n - k1;
         if (__ldcg(a.status + I_FAIL) >= 0) return;
         // ---- panel and right-hand side
-        const int nun = (rest + 7) / 8;                 // eight-row units; unit nun is the right-hand side
-        if (bx <= nun) {
+        // two rows a warp while every row has a warp of its own SM's (the row's chain of dependent
+        // operations bounds it: 3 us against 5), eight rows beyond (half the instructions a row)
+        const bool few = rest <= 2 * G * (CT / 32);
+        if (bx <= (few ? (rest + 1) / 2 : (rest + 7) / 8)) {
             for (int e = tid; e < CB * CB; e += CT) {
                 const int r = e >> 5, c = e & 31;
                 sm.B[r][c] = r < kb && c < r ? __ldcg(T + (size_t)(k0 + r) * n + k0 + c) : 0.0;
             }
             if (tid < CB) sm.rinv[tid] = tid < kb ? __ldcg(a.rd + k0 + tid) : 0.0;
             __syncthreads();
-            for (int u = bx + G * warp; u <= nun; u += G * (CT / 32)) {
-                const int row = k1 + u * 8 + (lane >> 2), q = lane & 3;
-                const bool ok = u < nun ? row < n : lane < 4;
-                double *p = u < nun ? T + (size_t)row * n + k0 : a.z + k0;
-                double s[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) s[i] = ok && q + 4 * i < kb ? __ldcg(p + q + 4 * i) : 0.0;
-                row_solve(s, sm.B, sm.rinv, kb, lane);
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                    if (ok && q + 4 * i < kb) p[q + 4 * i] = s[i];
-            }
+            if (few) panel_solve<16>(T, a.z, n, k0, kb, sm.B, sm.rinv);
+            else panel_solve<4>(T, a.z, n, k0, kb, sm.B, sm.rinv);
         }
         if (rest <= 0) break;
         if (!grid_barrier(a.bar, a.err, G)) return;
@@ -162,7 +195,7 @@ __global__ void __launch_bounds__(CT, 1) k_chol64(Chol64Args a) {
             for (int e = tid; e < CB * CB; e += CT) {
                 const int r = e >> 5, c = e & 31;
                 sm.B[r][c] = r < kn && c < kb ? __ldcg(P + (size_t)(k1 + r) * n + c) : 0.0;
-                sm.A[r][c] = r < kn && c <= r ? __ldcg(T + (size_t)(k1 + r) * n + k1 + c) : 0.0;
+                sm.A[r][c] = r < kn && c <= r ? __ldcg(T + (size_t)(k1 + r) * n + k1 + c) : (r == c ? 1.0 : 0.0);
             }
             if (tid < CB) sm.x[tid] = tid < kb ? __ldcg(a.z + k0 + tid) : 0.0;
             __syncthreads();
