@@ -28,6 +28,14 @@ int sampler_chains(const Sampler *sm);
 const unsigned long long *sampler_counts(const Sampler *sm);
 bool sampler_fp32(const Sampler *sm);
 
+// A step's words of one instance in pinned memory, written by its update kernel (five copies of a few
+// bytes per instance were five nodes of the batch's graph).
+struct BatchWords {
+    double scal[16], nrm[2];
+    unsigned long long counts[2];        // sampler: accepted, proposed
+    int status, err;                     // of the mixed solve
+};
+
 struct BatchInst {
     nqs_config_t cfg{};
     int sx = 0, sy = 0;
@@ -42,15 +50,11 @@ struct BatchInst {
     DevBuf<double> E, Ei, eps, O, gm, scal, delta, y, part, es;
     DevBuf<unsigned long long> move;
     MixedSys *mx = nullptr;
-    double *h = nullptr;      // pinned: scal[16], nrm[2]
-    int *hs = nullptr;        // pinned: mixed status, error word
-    unsigned long long *hc = nullptr;   // pinned: sampler counters (accepted, proposed)
+    BatchWords *h = nullptr;  // pinned: the step's words
     int fp64_fallback = 0, fp64_conv = 0;   // last step solved in FP64 after an FP32 breakdown
     ~BatchInst() {
         if (mx) mixed_sys_free(mx);
         if (h) cudaFreeHost(h);
-        if (hs) cudaFreeHost(hs);
-        if (hc) cudaFreeHost(hc);
     }
 };
 
@@ -89,8 +93,10 @@ __host__ __device__ inline bool mixed_broken(int status, const double *nrm) {
 // solve broke down or its kernels reported an error (decided by one thread: the
 // test's FP64 division and square root cost 16 cycles per warp instruction on this
 // GPU's FP64 pipe).
+// host, when given, receives the step's words.
 __global__ void k_batch_apply(double *params, const double *__restrict__ delta, long P, double lr, double *scal,
-                              const int *mstatus, const int *merr, const double *mnrm, int unconditional) {
+                              const int *mstatus, const int *merr, const double *mnrm, int unconditional,
+                              BatchWords *host, const unsigned long long *counts) {
     __shared__ double red[1024];
     __shared__ bool zero_s;
     if (threadIdx.x == 0) zero_s = !unconditional && (mixed_broken(mstatus[0], mnrm) || merr[0] != 0);
@@ -109,12 +115,22 @@ __global__ void k_batch_apply(double *params, const double *__restrict__ delta, 
         __syncthreads();
     }
     if (threadIdx.x == 0) scal[S_NORM2] = red[0];
+    if (!host) return;
+    if (threadIdx.x < 16) host->scal[threadIdx.x] = threadIdx.x == S_NORM2 ? red[0] : scal[threadIdx.x];
+    if (threadIdx.x < 2) {
+        host->nrm[threadIdx.x] = mnrm[threadIdx.x];
+        host->counts[threadIdx.x] = counts[threadIdx.x];
+    }
+    if (threadIdx.x == 0) {
+        host->status = mstatus[0];
+        host->err = merr[0];
+    }
 }
 
 bool enqueue_gated_apply(double *params, const double *delta, long P, double lr, double *scal, const int *mstatus,
                          const int *merr, const double *mnrm) {
     NQS_LAUNCH("apply_update");
-    k_batch_apply<<<1, 1024, 0, ctx().stream>>>(params, delta, P, lr, scal, mstatus, merr, mnrm, 0);
+    k_batch_apply<<<1, 1024, 0, ctx().stream>>>(params, delta, P, lr, scal, mstatus, merr, mnrm, 0, nullptr, nullptr);
     return NQS_CUDA(cudaGetLastError());
 }
 
@@ -135,16 +151,11 @@ static bool enqueue_back(BatchInst &b, cudaStream_t st) {
     {
         NQS_LAUNCH("apply_update");
         k_batch_apply<<<1, 1024, 0, st>>>(b.a->d_params.p, b.delta.p, b.P, b.cfg.learning_rate, b.scal.p,
-                                          mixed_sys_status(b.mx), mixed_sys_err(b.mx), mixed_sys_nrm(b.mx), 0);
+                                          mixed_sys_status(b.mx), mixed_sys_err(b.mx), mixed_sys_nrm(b.mx), 0, b.h,
+                                          sampler_counts(b.s));
     }
-    return NQS_CUDA(cudaMemcpyAsync(b.h, b.scal.p, 16 * sizeof(double), cudaMemcpyDeviceToHost, st)) &&
-           NQS_CUDA(cudaMemcpyAsync(b.h + 16, mixed_sys_nrm(b.mx), 2 * sizeof(double), cudaMemcpyDeviceToHost, st)) &&
-           NQS_CUDA(cudaMemcpyAsync(b.hs, mixed_sys_status(b.mx), sizeof(int), cudaMemcpyDeviceToHost, st)) &&
-           NQS_CUDA(cudaMemcpyAsync(b.hs + 1, mixed_sys_err(b.mx), sizeof(int), cudaMemcpyDeviceToHost, st)) &&
-           NQS_CUDA(cudaMemcpyAsync(b.hc, sampler_counts(b.s), 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                    st)) &&
-           NQS_CUDA(cudaMemcpyAsync(b.a->h_params, b.a->d_params.p, sizeof(double) * b.P, cudaMemcpyDeviceToHost,
-                                    st));
+    return NQS_CUDA(cudaGetLastError()) && NQS_CUDA(cudaMemcpyAsync(b.a->h_params, b.a->d_params.p, sizeof(double) * b.P,
+                                                                   cudaMemcpyDeviceToHost, st));
 }
 
 // Run `work(instance)` for every instance on the side streams (instance i on
@@ -392,9 +403,7 @@ nqs_gpu_batch_t *nqs_gpu_batch_create(const nqs_gpu_instance_t *in, int count) {
             !b->es.ensure(energy_scratch_doubles(b->Ns)) ||
             !NQS_CUDA(cudaMemset(b->es.p, 0, sizeof(double) * energy_scratch_doubles(b->Ns))) ||
             !NQS_CUDA(cudaMemcpy(b->move.p, &mv, sizeof(mv), cudaMemcpyHostToDevice)) ||
-            !NQS_CUDA(cudaMallocHost(&b->h, 18 * sizeof(double))) ||
-            !NQS_CUDA(cudaMallocHost(&b->hs, 2 * sizeof(int))) ||
-            !NQS_CUDA(cudaMallocHost(&b->hc, 2 * sizeof(unsigned long long)))) {
+            !NQS_CUDA(cudaMallocHost(&b->h, sizeof(BatchWords)))) {
             delete h;
             return nullptr;
         }
@@ -460,13 +469,14 @@ int nqs_gpu_batch_step(nqs_gpu_batch_t *h, nqs_sr_step_info_t *infos) {
     for (size_t i = 0; i < B.inst.size(); i++) {
         BatchInst *b = B.inst[i];
         b->fp64_fallback = 0;
-        if (!mixed_broken(b->hs[0], b->h + 16) || b->hs[1] != 0) continue;
+        if (!mixed_broken(b->h->status, b->h->nrm) || b->h->err != 0) continue;
         int conv = 0;
         if (minsr_fp64_delta(b->O.p, b->eps.p, b->Ns, b->P, b->cfg.sr_diag_shift, b->delta.p, &conv) != 0)
             return -1;
         k_batch_apply<<<1, 1024, 0, st>>>(b->a->d_params.p, b->delta.p, b->P, b->cfg.learning_rate, b->scal.p,
-                                          mixed_sys_status(b->mx), mixed_sys_err(b->mx), mixed_sys_nrm(b->mx), 1);
-        if (!NQS_CUDA(cudaMemcpyAsync(b->h + S_NORM2, b->scal.p + S_NORM2, sizeof(double), cudaMemcpyDeviceToHost,
+                                          mixed_sys_status(b->mx), mixed_sys_err(b->mx), mixed_sys_nrm(b->mx), 1,
+                                          nullptr, nullptr);
+        if (!NQS_CUDA(cudaMemcpyAsync(&b->h->scal[S_NORM2], b->scal.p + S_NORM2, sizeof(double), cudaMemcpyDeviceToHost,
                                       st)) ||
             !NQS_CUDA(cudaMemcpyAsync(b->a->h_params, b->a->d_params.p, sizeof(double) * b->P,
                                       cudaMemcpyDeviceToHost, st)) ||
@@ -481,20 +491,22 @@ int nqs_gpu_batch_step(nqs_gpu_batch_t *h, nqs_sr_step_info_t *infos) {
         BatchInst *b = B.inst[i];
         sampler_host_advance(b->s, b->Ns);
         memcpy(b->a->h_shadow, b->a->h_params, sizeof(double) * b->P);
-        if (b->hs[1]) failed = (int)i + 1;
+        if (b->h->err) failed = (int)i + 1;
         if (infos) {
             nqs_sr_step_info_t &f = infos[i];
-            f.mean_energy = b->h[S_EMEAN];
-            f.variance_energy = b->h[S_ESQ] - b->h[S_EMEAN] * b->h[S_EMEAN];
-            f.update_norm = sqrt(b->h[S_NORM2]) * b->cfg.learning_rate;
-            f.acceptance_ratio = b->hc[1] ? (double)b->hc[0] / (double)b->hc[1] : 0.0;
+            const double *sc = b->h->scal;
+            const unsigned long long *n = b->h->counts;
+            f.mean_energy = sc[S_EMEAN];
+            f.variance_energy = sc[S_ESQ] - sc[S_EMEAN] * sc[S_EMEAN];
+            f.update_norm = sqrt(sc[S_NORM2]) * b->cfg.learning_rate;
+            f.acceptance_ratio = n[1] ? (double)n[0] / (double)n[1] : 0.0;
             f.cg_iterations = 0;
-            f.converged = b->fp64_fallback ? b->fp64_conv : (!mixed_broken(b->hs[0], b->h + 16) && b->hs[1] == 0);
+            f.converged = b->fp64_fallback ? b->fp64_conv : (!mixed_broken(b->h->status, b->h->nrm) && b->h->err == 0);
         }
     }
     if (failed) {
         set_error("batch instance %d: %s", failed - 1,
-                  B.inst[failed - 1]->hs[1] == 2 ? "grid barrier timed out" : "tensor-core Gram timed out");
+                  B.inst[failed - 1]->h->err == 2 ? "grid barrier timed out" : "tensor-core Gram timed out");
         return -1;
     }
     return 0;

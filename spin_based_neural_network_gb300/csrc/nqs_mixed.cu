@@ -2363,15 +2363,31 @@ __global__ void k_center_split_t(double *O, int Ns, long P, const double *__rest
     }
 }
 
+// The words and vectors the Gram and the factor kernel expect, in one launch: status -1, error, barrier
+// and timer words 0, the padded FP32 vectors 0 (six memset nodes per system in a graph before).
+__global__ void k_solve_clear(int *status, int *err, unsigned *bar, unsigned long long *tm, float *rf, float *zf,
+                              int ldl) {
+    const int t = threadIdx.x;
+    if (t < 2) status[t] = -1;
+    if (t == 2) *err = 0;
+    if (t < 8) {
+        bar[t] = 0;
+        tm[t] = 0;
+    }
+    for (int i = t; i < ldl; i += blockDim.x) rf[i] = zf[i] = 0.f;
+}
+
 // Enqueue the whole mixed solve with no host synchronisation: centring and
 // split, tensor-core Gram, then the cooperative factor / inverse / refinement
 // kernel.  A broken factor is reported through status[0].
-// Front of the mixed solve: status words, centring and TF32 split, tensor-core Gram.
+// Front of the mixed solve: cleared words, centring and TF32 split, tensor-core Gram.
 static void enqueue_front(MixedWs &w, const MixedPlan &pl, double *O, const double *gm, int Ns, long P, double shift,
                           int passes, const CUtensorMap &mh, const CUtensorMap &ml, int *err, cudaStream_t st,
                           bool with_split = true) {
-    cudaMemsetAsync(w.status.p, 0xff, 2 * sizeof(int), st);
-    cudaMemsetAsync(err, 0, sizeof(int), st);
+    {
+        NQS_LAUNCH("solve_clear");
+        k_solve_clear<<<1, 1024, 0, st>>>(w.status.p, err, w.bar.p, w.tm.p, w.rf.p, w.zf.p, (pl.n + 31) / 32 * 32);
+    }
     if (!with_split) {
     } else if (pl.space == 0) {
         NQS_LAUNCH("center_split");
@@ -2452,14 +2468,6 @@ static FrArgs make_frargs(MixedWs &w, const MixedPlan &pl, double *O, const doub
     return fa;
 }
 
-// Zeroed words and vectors the factor / refinement kernel expects.
-static void enqueue_fr_clear(MixedWs &w, const FrArgs &fa, cudaStream_t st) {
-    cudaMemsetAsync(w.bar.p, 0, 8 * sizeof(unsigned), st);
-    cudaMemsetAsync(w.tm.p, 0, 8 * sizeof(unsigned long long), st);
-    cudaMemsetAsync(w.rf.p, 0, sizeof(float) * fa.ldl, st);
-    cudaMemsetAsync(w.zf.p, 0, sizeof(float) * fa.ldl, st);
-}
-
 static void enqueue_mixed(const MixedPlan &pl, double *O, const double *gm, const double *eps, int Ns, long P,
                           double shift, int sweeps, int passes, double *x, const CUtensorMap &mh,
                           const CUtensorMap &ml, int *err, cudaStream_t st, cudaEvent_t eps_ready, bool captured) {
@@ -2468,7 +2476,6 @@ static void enqueue_mixed(const MixedPlan &pl, double *O, const double *gm, cons
     // (in a graph: a node that waits for the event's record before each replay)
     if (eps_ready) NQS_CUDA(cudaStreamWaitEvent(st, eps_ready, captured ? cudaEventWaitExternal : 0));
     const FrArgs fa = make_frargs(w, pl, O, eps, Ns, P, shift, sweeps, x, err);
-    enqueue_fr_clear(w, fa, st);
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)ctx().sm_count);
     lc.blockDim = dim3(PS_THREADS);
@@ -3054,11 +3061,9 @@ bool mixed_sys_prepare(MixedSys *m, double *O, const double *gm, const double *e
     return true;
 }
 
-// Status words, centring + split (unless the operands are already split), Gram,
-// and the cleared words of the factor kernel.
+// Cleared words, centring + split (unless the operands are already split), Gram.
 void mixed_sys_front(MixedSys *m, cudaStream_t st, bool with_split) {
     enqueue_front(m->w, m->pl, m->O, m->gm, m->Ns, m->P, m->shift, m->passes, m->mh, m->ml, m->err.p, st, with_split);
-    enqueue_fr_clear(m->w, m->fa, st);
 }
 
 // Microseconds of the system's last timed solve, from its CTA 0 (0: it broke down).
