@@ -341,7 +341,176 @@ __device__ __forceinline__ unsigned long long gtimer() {
     return t;
 }
 
-// The 64 x 64 diagonal block, Cholesky and X = L^{-1} in one right-looking sweep over
+// 16 x 16 Cholesky and inverse by one warp: lane (i, h) = (lane & 15, lane >> 4) holds columns 2q + h
+// (q < 8) of row i of the symmetric block in s and of R (the identity on entry) in r.  Pivots in pairs:
+// with l10 and the two reciprocal roots formed by every lane, rows below take row_i -= al row_j +
+// be row_j+1 of S (columns past the pair) and of R (columns up to it), eight registers a lane in all.
+// Row i of L^{-1} goes to XD[i][0 .. 15].  Returns the first non-positive pivot or -1 (the entries are
+// then not used).
+constexpr int FP = 20;                                       // pitch of 16-float rows: float4 reads of 8 rows hit all banks
+__device__ __forceinline__ int warp_chol_inv16(float (&s)[8], float (*XD)[FP], int lane) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int i = lane & 15, h = lane >> 4;
+    float r[8], scale = 1.f;
+    int fail = -1;
+#pragma unroll
+    for (int q = 0; q < 8; q++) r[q] = 2 * q + h == i ? 1.f : 0.f;
+#pragma unroll
+    for (int jq = 0; jq < 8; jq++) {
+        const int j = 2 * jq;
+        const float p00 = __shfl_sync(ALL, s[jq], j), p10 = __shfl_sync(ALL, s[jq], j + 1),
+                    p11 = __shfl_sync(ALL, s[jq], j + 17);
+        const float a = __shfl_sync(ALL, s[jq], i), b = __shfl_sync(ALL, s[jq], i + 16);
+        const float inv0 = rsqrtf(p00), l10 = p10 * inv0;
+        const float d1 = fmaf(-l10, l10, p11), inv1 = rsqrtf(d1);
+        if (!(p00 > 0.f) && fail < 0) fail = j;
+        if (!(d1 > 0.f) && fail < 0) fail = j + 1;
+        const float li0 = a * inv0, li1 = fmaf(-li0, l10, b) * inv1;
+        const float be = i > j + 1 ? li1 * inv1 : 0.f;
+        const float al = i > j ? fmaf(-be, l10, li0) * inv0 : 0.f;
+        scale = i == j ? inv0 : i == j + 1 ? inv1 : scale;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const float x = q > jq ? s[q] : r[q];
+            const float x0 = __shfl_sync(ALL, x, j + 16 * h), x1 = __shfl_sync(ALL, x, j + 1 + 16 * h);
+            const float y = fmaf(-be, x1, fmaf(-al, x0, x));
+            if (q > jq) s[q] = y;
+            else r[q] = y;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) XD[i][2 * q + h] = r[q] * scale;
+    return fail;
+}
+
+__device__ __forceinline__ float dot4(float4 a, float4 b, float s) {
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+}
+
+// The 64 x 64 diagonal block, Cholesky and X = L^{-1} in one right-looking sweep over 16-column panels.
+// The matrix M is held by warps 2 .. 7 in registers (thread (ty, tx) = (tid / 16, tid % 16): rows
+// 4 ty + a, columns tx + 16 b), the columns past the panels as S, those up to them as R = I - L X.  Panel
+// p at k0 = 16 p:
+//   pivot   warp 0 updates the panel's diagonal block and factors and inverts it (XD) while the other
+//           warps still apply the panel before to M and publish the panel's columns of S and rows of
+//           R (P, one row of 16 per column or row of M);
+//   panel   V[c] = XD P[c] for the rows c of L below the panel (l_c) and the columns c of X up to it
+//           (x_c, also stored to X), a quarter of a row a thread;
+//   update  M[i][c] -= V[i] . V[c] for the rows i below the panel and c up to i's diagonal block.
+// Only the lower triangle of S is read (rows >= bs padded with the identity); its diagonal 16 x 16
+// blocks are overwritten.  X gets zeros above the diagonal.  Returns the first non-positive pivot column
+// below bs or -1 (the caller discards the block).  buf: 2881 floats, 16-byte aligned.
+// Bound by the chain of pivot pairs (two reciprocal roots and two shuffles each) of warp 0.  Measured:
+// the first block of a factor with its loads and stores 9.2 us; with four-column panels whose pivots
+// every thread factors for itself (block_chol_inv64_wide) 20.8 us, 1400 clocks a panel.
+__device__ int block_chol_inv64(float (*S)[BT + 1], float (*X)[BT + 1], int bs, float *buf) {
+    float (*V)[FP] = (float (*)[FP])buf, (*P)[FP] = (float (*)[FP])(buf + 64 * FP), (*XD)[FP] = (float (*)[FP])(buf + 128 * FP);
+    int *failp = (int *)(buf + 144 * FP);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, wb = w >> 1, tx = tid & 15, ty = tid >> 4;
+    float m[4][4];
+    {
+        const int c = tid >> 2;
+        if (c >= 16)
+#pragma unroll
+            for (int t = 0; t < 4; t++) P[c][(tid & 3) + 4 * t] = S[c][(tid & 3) + 4 * t];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const int i = 4 * ty + a, c = tx + 16 * b;
+            m[a][b] = b <= wb ? S[max(i, c)][min(i, c)] : 0.f;
+        }
+    if (w == 0) {
+        float s[8];
+        const int i = lane & 15, h = lane >> 4;
+#pragma unroll
+        for (int q = 0; q < 8; q++) s[q] = S[max(i, 2 * q + h)][min(i, 2 * q + h)];
+        const int f = warp_chol_inv16(s, XD, lane);
+        if (lane == 0) *failp = f >= 0 && f < bs ? f : -1;
+    }
+#pragma unroll 1
+    for (int p = 0; p < 4; p++) {
+        const int k0 = 16 * p, k1 = k0 + 16;
+        __syncthreads();
+        {
+            const int c = tid >> 2, q = tid & 3;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (wb == p) {
+#pragma unroll
+                for (int t = 0; t < 4; t++) v[t] = XD[q + 4 * t][c & 15];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 16; k += 4) {
+                    const float4 x = *(const float4 *)&P[c][k];
+#pragma unroll
+                    for (int t = 0; t < 4; t++) v[t] = dot4(*(const float4 *)&XD[q + 4 * t][k], x, v[t]);
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                V[c][q + 4 * t] = v[t];
+                X[k0 + q + 4 * t][c] = wb <= p ? v[t] : 0.f;
+            }
+        }
+        if (p == 3) break;
+        __syncthreads();
+        if (w == 0) {
+            // the next panel's diagonal block (updated by the panels before this one in S) and its factor
+            const int i = lane & 15, h = lane >> 4;
+            float s[8];
+            float4 vi[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) vi[k] = *(const float4 *)&V[k1 + i][4 * k];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int c = 2 * q + h;
+                float d = 0.f;
+#pragma unroll
+                for (int k = 0; k < 4; k++) d = dot4(vi[k], *(const float4 *)&V[k1 + c][4 * k], d);
+                s[q] = S[k1 + max(i, c)][k1 + min(i, c)] - d;
+            }
+            const int f = warp_chol_inv16(s, XD, lane);
+            if (lane == 0 && f >= 0 && k1 + f < bs && *failp < 0) *failp = k1 + f;
+        } else if (wb > p) {
+            float acc[4][4] = {};
+#pragma unroll
+            for (int k = 0; k < 16; k += 4) {
+                float4 vi[4];
+#pragma unroll
+                for (int a = 0; a < 4; a++) vi[a] = *(const float4 *)&V[4 * ty + a][k];
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    if (b <= wb) {                           // (warp-uniform)
+                        const float4 vc = *(const float4 *)&V[tx + 16 * b][k];
+#pragma unroll
+                        for (int a = 0; a < 4; a++) acc[a][b] = dot4(vi[a], vc, acc[a][b]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+#pragma unroll
+                for (int a = 0; a < 4; a++) m[a][b] = (b == p ? 0.f : m[a][b]) - acc[a][b];
+                if (wb == p + 1 && b <= p)                   // rows of R
+                    *(float4 *)&P[tx + 16 * b][4 * (ty & 3)] = make_float4(m[0][b], m[1][b], m[2][b], m[3][b]);
+            }
+            // column block b of m, by selects (an index would put m into local memory)
+            auto pick = [&](int a, int b) { return b == 1 ? m[a][1] : b == 2 ? m[a][2] : m[a][3]; };
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                if (wb > p + 1) P[4 * ty + a][tx] = pick(a, p + 1);             // columns of S
+                if (wb == p + 2) S[4 * ty + a][tx + 16 * wb] = pick(a, p + 2);  // the diagonal block after the next
+            }
+        }
+    }
+    __syncthreads();
+    const int fail = *failp;
+    __syncthreads();
+    return fail;
+}
+
+// The halves of the 128-wide blocks: as block_chol_inv64, in one right-looking sweep over
 // four-column panels with the block in registers: thread (w, l) = (tid / 32, tid % 32)
 // holds rows i = w + 8u (u < 8) and columns c = l + 32v (v < 2) of S and of
 // R = I - L X (forward substitution of L X = I, right-looking).  At panel j0 the owners
@@ -355,8 +524,10 @@ __device__ __forceinline__ unsigned long long gtimer() {
 // Entries above the diagonal of S take values nothing reads.  S (rows >= bs padded with
 // the identity) is read once; X (zeros above the diagonal) is written to X.  Returns the
 // first non-positive pivot column below bs or -1 (the sweep goes on with a unit pivot; the
-// caller discards the block).  buf: 1024 floats.
-__device__ int block_chol_inv64(const float (*S)[BT + 1], float (*X)[BT + 1], int bs, float *buf) {
+// caller discards the block).  buf: 1024 floats.  Measured at order 8192: 46 us a block
+// with all its steps, as with the 16-column sweep, and the step 12.9 ms, 13.05 ms with that (this kernel
+// is short of registers and spills more beside the longer code).
+__device__ int block_chol_inv64_wide(const float (*S)[BT + 1], float (*X)[BT + 1], int bs, float *buf) {
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     float s[8][2], r[8][2];
 #pragma unroll
@@ -534,7 +705,7 @@ __device__ int block_chol_inv128(float (*S)[BT + 1], float (*X)[BT + 1], int bs,
     const Block S21 = (Block)&S[64][0], S22 = (Block)&S[64][64], X12 = (Block)&X[0][64], X21 = (Block)&X[64][0],
                 X22 = (Block)&X[64][64];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    int f = block_chol_inv64(S, X, min(bs, 64), buf);
+    int f = block_chol_inv64_wide(S, X, min(bs, 64), buf);
     if (f >= 0) return f;
     __syncthreads();
     float acc[4][4];
@@ -562,7 +733,7 @@ __device__ int block_chol_inv128(float (*S)[BT + 1], float (*X)[BT + 1], int bs,
 #pragma unroll
         for (int v = 0; v < 4; v++) S22[ty + 16 * u][tx + 16 * v] -= acc[u][v];
     __syncthreads();
-    f = block_chol_inv64(S22, X22, max(bs - 64, 0), buf);
+    f = block_chol_inv64_wide(S22, X22, max(bs - 64, 0), buf);
     if (f >= 0) return 64 + f;
     __syncthreads();
     clear();
@@ -1252,7 +1423,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
     const int gtid = bx * PS_THREADS + tid, gthreads = G * PS_THREADS;
     const int gwarp = bx * (PS_THREADS / 32) + (tid >> 5), gwarps = G * (PS_THREADS / 32);
     const int nb = (n + BD - 1) / BD;
-    __shared__ float tmpb[3 * 1024];
+    __shared__ __align__(16) float tmpb[3 * 1024];
     unsigned long long tacc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const bool timing = a.tm != nullptr && bx == 0 && tid == 0;
     unsigned long long tstart = timing ? gtimer() : 0, tprev = tstart;
@@ -2262,14 +2433,16 @@ struct FrMaps {
     CUtensorMap m[3];
 };
 
+// A kernel per block width: with both bodies in one the 64-wide one runs slower (the 4x4 Heisenberg step
+// of 4096 samples takes 831 us instead of 799 us) and both spill.
+template <int BD>
 __global__ void __launch_bounds__(PS_THREADS, 1) k_factor_refine(FrArgs a, const __grid_constant__ FrMaps maps,
                                                                 int have_maps) {
     __shared__ uint64_t mbar[5];
     __shared__ uint32_t slot;
     TcState ts;
     tc_setup(ts, mbar, &slot, a.err);
-    if (a.bd == BD_LARGE) fr_body<BD_LARGE>(a, blockIdx.x, gridDim.x, ts, have_maps ? maps.m : nullptr);
-    else fr_body<BD_SMALL>(a, blockIdx.x, gridDim.x, ts);
+    fr_body<BD>(a, blockIdx.x, gridDim.x, ts, have_maps ? maps.m : nullptr);
     tc_teardown(ts);
 }
 
@@ -2491,7 +2664,7 @@ static void enqueue_mixed(const MixedPlan &pl, double *O, const double *gm, cons
         const int have = fa.bd == BD_LARGE && make_map(&maps.m[0], w.uh.p, fa.n + TT, BD_LARGE) &&
                          make_map(&maps.m[1], w.ul.p, fa.n + TT, BD_LARGE) && make_map(&maps.m[2], w.T.p, fa.n, fa.ldl);
         NQS_LAUNCH("factor_refine");
-        cudaLaunchKernelEx(&lc, k_factor_refine, fa, maps, have);
+        cudaLaunchKernelEx(&lc, fa.bd == BD_LARGE ? k_factor_refine<BD_LARGE> : k_factor_refine<BD_SMALL>, fa, maps, have);
     }
 }
 
@@ -2552,13 +2725,15 @@ static bool ensure_attrs() {
     static bool attr = false;
     if (attr) return true;
     if (!NQS_CUDA(cudaFuncSetAttribute(k_gram_tf32_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM)) ||
-        !NQS_CUDA(cudaFuncSetAttribute(k_factor_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM)) ||
+        !NQS_CUDA(cudaFuncSetAttribute(k_factor_refine<BD_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM)) ||
+        !NQS_CUDA(cudaFuncSetAttribute(k_factor_refine<BD_LARGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM)) ||
         !NQS_CUDA(cudaFuncSetAttribute(k_factor_refine_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM)))
         return false;
-    int per_sm = 0;
-    if (!NQS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_factor_refine, PS_THREADS, PS_SMEM)))
+    int small = 0, large = 0;
+    if (!NQS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small, k_factor_refine<BD_SMALL>, PS_THREADS, PS_SMEM)) ||
+        !NQS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&large, k_factor_refine<BD_LARGE>, PS_THREADS, PS_SMEM)))
         return false;
-    if (per_sm < 1) {
+    if (small < 1 || large < 1) {
         set_error("factor / refinement kernel does not fit on an SM");
         return false;
     }
