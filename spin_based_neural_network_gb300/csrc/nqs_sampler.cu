@@ -4,11 +4,13 @@
 // launch the warp rebuilds theta_h = b_h + sum_i W_hi s_i in registers (lane =
 // hidden unit) and then runs its proposals with O(M) incremental updates:
 // a single flip at u or an exchange on bond (u, v) changes theta by one or two
-// weight columns, the acceptance needs only Re log(2 cosh theta') (3 FP64
-// transcendentals per hidden unit) and one warp butterfly.  Random numbers are
-// computed redundantly by all lanes (xorshift64 state replicated in registers,
-// or counter-based Philox4x32-10 keyed by (seed, chain) with counter = move
-// index), so no lane ever waits on another for them.
+// weight columns.  The FP64 Philox chains carry r_h = exp(-2 theta_h) instead and
+// accept on a product of (L + X r) / (1 + r) factors (k_sample_rbm_ratio,
+// k_sample_rbm_pair); the compat chain and chains whose theta leaves the range of
+// exp need Re log(2 cosh theta') (3 FP64 transcendentals per hidden unit).  One warp
+// butterfly either way.  Random numbers are computed redundantly by all lanes
+// (xorshift64 state replicated in registers, or counter-based Philox4x32-10 keyed by
+// (seed, chain) with counter = move index), so no lane ever waits on another for them.
 //
 // Compat mode (one chain, xorshift64) replays the upstream chain of
 // src/nqs/nqs_sampler.c:86-117 proposal for proposal: same site choice
