@@ -59,8 +59,7 @@ struct GridSum {
 // Sum over the block in a fixed order (thread 0 holds it): the tree of each warp's values (lane l
 // takes lane l + 16, 8, 4, 2, 1), then the warps in turn.  One warp forms the trees of all eight from
 // shared memory, 9 FP64 instructions where a shuffle tree in every warp takes 40.
-__device__ __forceinline__ double block_sum(double v) {
-    __shared__ double red[2][ED_THREADS];
+__device__ __forceinline__ double block_sum(double v, double (*red)[ED_THREADS]) {
     red[0][threadIdx.x] = v;
     __syncthreads();
     double t = 0.0;
@@ -84,10 +83,11 @@ __device__ __forceinline__ double block_sum(double v) {
 // thread 0 calls fin(total).  So the kernels that use the sum read one number instead of every
 // block summing all partials (at 2^18 states that, with its square root and division in every
 // warp, was most of their time).  *ticket is zero before the first launch and again after each.
+// red: two rows of a block's values in shared memory.
 template <typename F>
-__device__ __forceinline__ void grid_sum(double v, double *part, unsigned *ticket, F fin) {
+__device__ __forceinline__ void grid_sum(double v, double *part, unsigned *ticket, double (*red)[ED_THREADS], F fin) {
     __shared__ bool last;
-    v = block_sum(v);
+    v = block_sum(v, red);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = v;
         __threadfence();
@@ -98,7 +98,7 @@ __device__ __forceinline__ void grid_sum(double v, double *part, unsigned *ticke
     __threadfence();
     double t = 0.0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += ED_THREADS) t += __ldcg(part + i);
-    t = block_sum(t);
+    t = block_sum(t, red);
     if (threadIdx.x == 0) {
         *ticket = 0;
         fin(t);
@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(ED_THREADS) k_heis_matvec(const double *__rest
         y[s] = val;
         dot = fma(xs, val, dot);
     }
-    if (R.part) grid_sum(dot, R.part, R.ticket, [&](double t) { *R.out = t; });
+    __shared__ double red[2][ED_THREADS];
+    if (R.part) grid_sum(dot, R.part, R.ticket, red, [&](double t) { *R.out = t; });
 }
 
 // y[s] = scale * sum_e chi[e] x[pi_e(s)] over m group elements, pi_e(s) = OR_c tab[e][c][nibble c
@@ -209,7 +210,11 @@ __global__ void __launch_bounds__(ED_THREADS) k_perm_sum(const double *__restric
         y[s] = v;
         nrm = fma(v, v, nrm);
     }
-    if (R.part) grid_sum(nrm, R.part, R.ticket, [&](double t) { *R.out = sqrt(t); });
+    if (!R.part) return;
+    // in the tables' shared memory, which bounds the blocks per SM (2^27 states, p6m E2: 12 % slower
+    // with 4 KB of its own)
+    __syncthreads();
+    grid_sum(nrm, R.part, R.ticket, (double (*)[ED_THREADS])ed_smem, [&](double t) { *R.out = sqrt(t); });
 }
 
 // out bit i of A x = parity(rows[i] & x): one GF(2) matrix of 64 rows.
@@ -298,7 +303,8 @@ __global__ void __launch_bounds__(ED_THREADS) k_sumsq(const double *__restrict__
     double t = 0.0;
     const unsigned stride = gridDim.x * ED_THREADS;
     for (unsigned s = blockIdx.x * ED_THREADS + threadIdx.x; s < dim; s += stride) t = fma(x[s], x[s], t);
-    grid_sum(t, R.part, R.ticket, [&](double q) { *R.out = sqrt(q); });
+    __shared__ double red[2][ED_THREADS];
+    grid_sum(t, R.part, R.ticket, red, [&](double q) { *R.out = sqrt(q); });
 }
 
 // x *= 1 / n when n = ||x|| > 0 (src/mps/lanczos.c:1104-1105).
@@ -590,7 +596,8 @@ bool launch_perm_pass(const ProjPlan &P, int pass, const double *x, double *y, u
     int off = 0;
     for (int k = 0; k < pass; k++) off += P.size[k];
     const int m = P.size[pass];
-    const size_t smem = (size_t)m * (ED_TAB * sizeof(unsigned) + sizeof(double));
+    const size_t smem = std::max((size_t)m * (ED_TAB * sizeof(unsigned) + sizeof(double)),
+                                 2 * ED_THREADS * sizeof(double));      // (and the norm's two rows)
     NQS_LAUNCH("ed_project_pass");
     k_perm_sum<<<ed_grid(dim), ED_THREADS, smem, st>>>(x, y, dim, m, P.tab.p + (size_t)off * ED_TAB,
                                                        P.chi.p + off, scale, R, popc);
