@@ -3019,10 +3019,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_rows(CgArgs a, int R) {
             if (lane == 0) up[w] = x0;
         }
         __syncthreads();
-        if (tid < items) {
-            double v = up[tid * S];
-            for (int q = 1; q < S; q++) v += up[tid * S + q];
-            us[tid] = v;
+        for (int i = tid; i < items; i += PS_THREADS) {
+            double v = up[i * S];
+            for (int q = 1; q < S; q++) v += up[i * S + q];
+            us[i] = v;
         }
         __syncthreads();
 #pragma unroll
