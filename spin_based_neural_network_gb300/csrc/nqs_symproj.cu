@@ -155,7 +155,11 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
                 if (CPLX) xi += sflip(a.wti[(long)i * M + h], pb, i);
             }
             const bool n = xr < 0.0;
-            const double em1 = expm1(-2.0 * fabs(xr)) + (xr - xr), e = 1.0 + em1;   // NaN for an infinite theta
+            // r is kept for factors X of up to exp(350), so it has to be exact to its own size: from exp; the
+            // sums 1 + r and 1 - r take it from expm1.  (NaN for an infinite theta)
+            const double em1 = VALS == 1 ? 0.0 : expm1(-2.0 * fabs(xr)) + (xr - xr);
+            const double e = VALS == 1 ? exp(-2.0 * fabs(xr)) + (xr - xr) : 1.0 + em1;
+            const double ep1 = VALS == 1 ? 1.0 + e : 2.0 + em1;
             lr += fabs(xr);
             if (CPLX) {
                 li += n ? -xi : xi;
@@ -163,7 +167,7 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
                 sincos(xi, &sn, &cs);
                 const double es = e * sn, u = 2.0 * es * sn;          // e (1 - cos 2y)
                 const double v = (n ? 2.0 : -2.0) * es * cs;          // Im r
-                const double2 d = make_double2((2.0 + em1) - u, v);   // 1 + r
+                const double2 d = make_double2(ep1 - u, v);           // 1 + r
                 if (VALS == 1) val[h] = make_double2(e - u, v);
                 if (VALS == 2) {
                     const double f = (n ? -1.0 : 1.0) / fma(d.x, d.x, d.y * d.y);
@@ -173,8 +177,8 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
                 P = cmul(P, d);
             } else {
                 if (VALS == 1) val[h] = make_double2(e, 0.0);
-                if (VALS == 2) val[h] = make_double2((n ? em1 : -em1) / (2.0 + em1), 0.0);
-                P.x *= 2.0 + em1;
+                if (VALS == 2) val[h] = make_double2((n ? em1 : -em1) / ep1, 0.0);
+                P.x *= ep1;
             }
         }
         if (VALS == 1) {
