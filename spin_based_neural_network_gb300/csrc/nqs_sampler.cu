@@ -231,11 +231,20 @@ __global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A)
 // 512 chains x 144 exchange proposals, 6x6 complex
 // RBM, 72 units: 174 us against 1161 us (log cosh of every unit).
 //
-// Range: chains whose weights could drive r_h, |1 + r_h|^2 or K out of a double's range (that need
-// |theta_h| <= 300, or 150 if complex, for every configuration and |sum Re D + visible| <= 250 for
-// every move) leave done[c] = 0 and are run by k_sample_generic, through log|psi|.
+// Range: chains whose weights could drive r_h, g_h, |1 + r_h|^2 or K out of a double's range (that need
+// |theta_h| <= 300, or 150 if complex, for every configuration, and |2 Re D_h| <= 700 for every unit and
+// |sum Re D + visible| <= 250 of every move) leave done[c] = 0 and are run by k_sample_generic,
+// through log|psi|.
 constexpr float kThetaRange = 300.f;
-constexpr double kMoveRange = 250.0;
+constexpr double kMoveRange = 250.0, kFactorRange = 700.0;
+
+// |Re theta_h| within range for every configuration (false for NaN too); the bound in FP32
+template <bool CPLX>
+__device__ __forceinline__ bool theta_in_range(const DevAnsatz &a, int h) {
+    float re = fabsf((float)a.p[a.N + h]);
+    for (int i = 0; i < a.N; i++) re += fabsf(a.w32[(long)i * a.M + h].x);
+    return re <= (CPLX ? 0.5f : 1.f) * kThetaRange;
+}
 
 __device__ __forceinline__ void chain_move(const SampleArgs &S, int move, int m, int &u, int &v) {
     if (move == NQS_GPU_MOVE_EXCHANGE) {
@@ -259,6 +268,7 @@ __global__ void __launch_bounds__(128) k_chain_tables(SampleArgs S, DevAnsatz a,
     int u, v;
     chain_move(S, move, m, u, v);
     double sum = 0.0;
+    bool ok = true;
     for (int h = lane; h < M; h += 32) {
         double x = a.wtr[(long)u * M + h], y = 0.0;
         if (v >= 0) x -= a.wtr[(long)v * M + h];
@@ -267,6 +277,7 @@ __global__ void __launch_bounds__(128) k_chain_tables(SampleArgs S, DevAnsatz a,
             if (v >= 0) y -= a.wti[(long)v * M + h];
         }
         sum += 2.0 * x;
+        ok = ok && fabs(4.0 * x) <= kFactorRange;
         const double gp = exp(4.0 * x), gm = exp(-4.0 * x);
         double *t = tab + ((size_t)m * (M + 1) + h) * W;
         if (CPLX) {
@@ -282,12 +293,13 @@ __global__ void __launch_bounds__(128) k_chain_tables(SampleArgs S, DevAnsatz a,
         }
     }
     sum = warp_sum(sum) + 2.0 * (a.p[u] - (v >= 0 ? a.p[v] : 0.0));
+    ok = __all_sync(0xffffffffu, ok);
     if (lane == 0) {
         double *t = tab + ((size_t)m * (M + 1) + M) * W;
         t[0] = exp(CPLX ? -2.0 * sum : -sum);
         t[CPLX ? 2 : 1] = exp(CPLX ? 2.0 * sum : sum);
         if (CPLX) t[1] = t[3] = 0.0;
-        range_ok[m] = fabs(sum) <= kMoveRange;
+        range_ok[m] = ok && fabs(sum) <= kMoveRange;
     }
 }
 
@@ -318,19 +330,10 @@ k_sample_rbm_ratio(SampleArgs S, DevAmp A, const double *__restrict__ tab, const
     const int c = blockIdx.x * kSW + (threadIdx.x >> 5);
     if (c >= S.C) return;
     const DevAnsatz &a = A.a;
-    const int M = a.M, N = a.N;
+    const int M = a.M;
     uint64_t s = S.bits[c];
-    // range: bound of |Re theta_h| over all configurations (FP32), and the moves' factors
     bool ok = true;
-#pragma unroll
-    for (int j = 0; j < J; j++) {
-        const int h = lane + 32 * j;
-        if (h < M) {
-            float bound = fabsf((float)a.p[N + h]);
-            for (int i = 0; i < N; i++) bound += fabsf(a.w32[(long)i * M + h].x);
-            ok = ok && bound <= (CPLX ? 0.5f : 1.f) * kThetaRange;   // false for NaN too
-        }
-    }
+    for (int h = lane; h < M; h += 32) ok = ok && theta_in_range<CPLX>(a, h);
     for (int m = lane; m < nm; m += 32) ok = ok && range_ok[m] != 0;
     ok = __all_sync(0xffffffffu, ok);
     if (lane == 0) done[c] = ok;
@@ -508,18 +511,13 @@ k_sample_rbm_pair(SampleArgs S, DevAmp A, const double *__restrict__ tab, const 
     const int lane = threadIdx.x & 31, sl = lane & 15, half = lane >> 4;
     const int c = blockIdx.x * kSW + (threadIdx.x >> 5);
     const DevAnsatz &a = A.a;
-    const int M = a.M, N = a.N;
+    const int M = a.M;
     for (int e = threadIdx.x; e < nm * (M + 1) * W; e += blockDim.x) rows[e] = tab[e];
     __syncthreads();
     if (c >= S.C) return;
     const bool own = sl < M;
     uint64_t s = S.bits[c];
-    bool ok = true;
-    if (own) {
-        float bound = fabsf((float)a.p[N + sl]);
-        for (int i = 0; i < N; i++) bound += fabsf(a.w32[(long)i * M + sl].x);
-        ok = bound <= (CPLX ? 0.5f : 1.f) * kThetaRange;
-    }
+    bool ok = !own || theta_in_range<CPLX>(a, sl);
     for (int m = lane; m < nm; m += 32) ok = ok && range_ok[m] != 0;
     ok = __all_sync(0xffffffffu, ok);
     if (lane == 0) done[c] = ok;
