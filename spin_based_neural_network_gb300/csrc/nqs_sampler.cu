@@ -233,17 +233,21 @@ __global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A)
 //
 // Range: chains whose weights could drive r_h, g_h, |1 + r_h|^2 or K out of a double's range (that need
 // |theta_h| <= 300, or 150 if complex, for every configuration, and |2 Re D_h| <= 700 for every unit and
-// |sum Re D + visible| <= 250 of every move) leave done[c] = 0 and are run by k_sample_generic,
-// through log|psi|.
+// |sum Re D + visible| <= 250 of every move) or are not finite leave done[c] = 0 and are run by
+// k_sample_generic, through log|psi|.
 constexpr float kThetaRange = 300.f;
 constexpr double kMoveRange = 250.0, kFactorRange = 700.0;
 
-// |Re theta_h| within range for every configuration (false for NaN too); the bound in FP32
+// |Re theta_h| within range for every configuration and Im theta_h finite (false for NaN too); bounds in FP32
 template <bool CPLX>
 __device__ __forceinline__ bool theta_in_range(const DevAnsatz &a, int h) {
-    float re = fabsf((float)a.p[a.N + h]);
-    for (int i = 0; i < a.N; i++) re += fabsf(a.w32[(long)i * a.M + h].x);
-    return re <= (CPLX ? 0.5f : 1.f) * kThetaRange;
+    float re = fabsf((float)a.p[a.N + h]), im = CPLX ? fabsf((float)a.p[crbm_pr(a) + a.N + h]) : 0.f;
+    for (int i = 0; i < a.N; i++) {
+        const float2 w = a.w32[(long)i * a.M + h];
+        re += fabsf(w.x);
+        if (CPLX) im += fabsf(w.y);
+    }
+    return re <= (CPLX ? 0.5f : 1.f) * kThetaRange && im <= 3e38f;
 }
 
 __device__ __forceinline__ void chain_move(const SampleArgs &S, int move, int m, int &u, int &v) {

@@ -1,5 +1,6 @@
 """FP64 Philox chains at the edges of the product form's range, against the oracle's chains, sample for
-sample: weights whose factors overflow a double while the theta and the moves' sums stay small."""
+sample: weights whose factors overflow a double while the theta and the moves' sums stay small, and
+parameters that are not finite."""
 import numpy as np
 import pytest
 
@@ -48,3 +49,16 @@ def test_opposite_units(nqs, kind, M, w):
         W[2:, :] *= 0.2
     for exchange in (False, True):
         compare(nqs, kind, 4, 1, M, fill, exchange)
+
+
+@pytest.mark.parametrize("M", [5, 20])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("part,imag", [("bias", False), ("bias", True), ("weight", False), ("weight", True), ("visible", True)])
+def test_parameters_that_are_not_finite(nqs, M, bad, part, imag):
+    N = 8
+    k = {"visible": 3, "bias": N + 2, "weight": N + M + 2 * N + 3}[part] + (N + M + M * N if imag else 0)
+
+    def fill(p):
+        p[k] = bad
+    for exchange in (False, True):
+        compare(nqs, O.OR_CRBM, 4, 2, M, fill, exchange)
