@@ -1833,15 +1833,13 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
             // the update of R by block row kb of X
             {
                 const int bs1 = min(BD, rest);                  // order of the next diagonal block
-                if (bx == 0 && tma_tiles) {
-                    // trailing tile 0 is the next diagonal block
-                    if (!trailing_tiles_tma(ts, mu, a.T, n, ldl, k1, 0, 1, 1)) return;
-                    factor_diag(kb + 1, -1, 0);
-                } else if (bx == 0 && BD == 64) {
+                if (bx == 0 && BD == 64) {
                     factor_diag(kb + 1, k0, bs);                // the update fused into the block's load
                 } else if (bx == 0) {
                     // D -= U_kb^T U_kb on the lower 64 x 64 tiles of the next diagonal block, FP32
-                    // from U (= L^T, the upper triangle rows k0 .. k0 + bs - 1 of T)
+                    // from U (= L^T, the upper triangle rows k0 .. k0 + bs - 1 of T).  (Not as a tile on
+                    // the tensor cores: three TF32 products over these 128 columns are 6 times as far
+                    // from 64 bits, rms 1.9e-7 against 2.8e-8 of the rows' norms.)
                     const float *U = a.T + (size_t)k0 * ldl;
                     for (int ti = 0; ti * GT < bs1; ti++)
                         for (int tj = 0; tj <= ti; tj++) {
@@ -1861,7 +1859,7 @@ __device__ __forceinline__ void fr_body(const FrArgs &a, const int bx, const int
                 }
                 const int ntt = (rest + TT - 1) / TT, ntiles = ntt * (ntt + 1) / 2;
                 const int ncr = blocked ? 0 : (k1 + TT - 1) / TT, nall = ntiles + ntt * ncr;
-                // (from tile 1 when CTA 0 has taken tile 0)
+                // (128-wide: tile 0 is the next diagonal block, all of it CTA 0's)
                 const int t0 = (G > 1 ? bx - 1 : 0) + (tma_tiles && (bx > 0 || G == 1) ? 1 : 0), dt = G > 1 ? G - 1 : 1;
                 auto job = [&](int t) -> TileJob {
                     if (t >= ntiles) {
