@@ -215,8 +215,8 @@ bool fp32_mlp_capable(const DevAmp &A);    // MLP with width <= 128 and FP32 tab
 bool launch_gradient(const DevAnsatz &a, const uint64_t *bits, int B, int mode, double *O, double *Oi);
 bool launch_symproj_gradient(const DevAmp &A, const uint64_t *bits, int B, double *O);
 bool launch_symproj_gradient_complex(const DevAmp &A, const uint64_t *bits, int B, double *O, double *Oi);
-// symmetry-projected RBM / complex RBM programs (nqs_symproj.cu); *done (device) = 0 leaves the
-// energies to the generic kernel
+// symmetry-projected RBM / complex RBM programs (nqs_symproj.cu); done[b] (device) = 0 leaves the energy
+// of configuration b to the generic kernel
 bool sym_log_amp_capable(const DevAmp &A);
 bool launch_sym_log_amp(const DevAmp &A, const uint64_t *bits, int B, double *la, double *ar);
 bool sym_gradient_capable(const DevAmp &A);

@@ -690,11 +690,10 @@ k_local_rbm32(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doub
 __global__ void __launch_bounds__(32 * kWarps)
 k_local_generic(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, double *Er, double *Ei,
                 const int *done) {
-    if (done && *done) return;                             // the projected product form has run
     extern __shared__ double sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * kWarps + warp;
-    if (b >= B) return;
+    if (b >= B || (done && done[b])) return;               // done: the projected product form has run
     double *scr = sm + warp * 4 * A.a.M;
     const uint64_t s = bits[b];
     const int N = A.a.N;

@@ -31,6 +31,20 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
 }
 
+// prod (1 + r) runs down to 0.03^M and below (hidden biases near i pi / 2, where cosh acts as i sinh), past
+// the range of a double at M = 144: log-amplitudes and gradients take factors 2^512 out of it below
+// 2^-400 (e counts them), energies leave a configuration with an element below kProdMin to the logarithms.
+__device__ __forceinline__ void lift(double2 &P, int &e) {
+    if (fmax(fabs(P.x), fabs(P.y)) < 0x1p-400) {
+        P.x *= 0x1p512;
+        P.y *= 0x1p512;
+        e++;
+    }
+}
+// No product of the energies that matters in the sum underflows above it: a partial product below 1e-308 times
+// the others' 2^256 e^350 at most is 1e-19 of 1e-60.
+constexpr double kProdMin = 1e-60;
+
 __host__ __device__ inline int pair_rows(int N) { return N * (N - 1) / 2 + N; }
 // row of the pair i < j, or of the single site i (j < 0)
 __device__ __forceinline__ int pair_row(int N, int i, int j) {
@@ -139,6 +153,7 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
     unsigned char *neg = smb + L.neg + 32 * (size_t)g;              // bit h % 8 of byte h / 8
     double lr = 0.0, li = 0.0;
     double2 P = make_double2(1.0, 0.0);
+    int pe = 0;
     if (in)
         for (int i = sl; i < N; i += 8) {
             lr += sflip(a.p[i], pb, i);
@@ -175,6 +190,7 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
                     val[h] = make_double2(t.x * f, t.y * f);
                 }
                 P = cmul(P, d);
+                if (VALS != 1) lift(P, pe);
             } else {
                 if (VALS == 1) val[h] = make_double2(e, 0.0);
                 if (VALS == 2) val[h] = make_double2((n ? em1 : -em1) / ep1, 0.0);
@@ -193,7 +209,12 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
         else P.x *= x;
         lr += __shfl_xor_sync(0xffffffffu, lr, o);
         if (CPLX) li += __shfl_xor_sync(0xffffffffu, li, o);
+        if (CPLX && VALS != 1) {
+            pe += __shfl_xor_sync(0xffffffffu, pe, o);
+            lift(P, pe);
+        }
     }
+    if (pe > 0) lr -= (double)pe * 354.89135644669200;              // 512 ln 2
     if (in && sl == 0) {
         ((double *)(smb + L.lp))[g] = lr;
         ((double *)(smb + L.ag))[g] = li;
@@ -202,23 +223,28 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
 }
 
 // Weights w_g = chi_g exp(lp_g - max + i arg_g) by one warp, an element a lane (inner Marshall layers
-// included; INV: pinv becomes 1 / prod (1 + r)); returns max and sum_g w_g (all lanes).
+// included; INV: pinv becomes 1 / prod (1 + r), small says that one of these is below kProdMin or NaN);
+// returns max and sum_g w_g (all lanes).
 template <bool INV, bool CPLX>
-__device__ __forceinline__ double sym_weights(const DevAmp &A, unsigned char *smb, const SymSmem &L, double2 &sum) {
+__device__ __forceinline__ double sym_weights(const DevAmp &A, unsigned char *smb, const SymSmem &L, double2 &sum,
+                                              bool *small = nullptr) {
     const int lane = threadIdx.x & 31;
     double *lp = (double *)(smb + L.lp), *ag = (double *)(smb + L.ag);
     double2 *w = (double2 *)(smb + L.w), *pinv = (double2 *)(smb + L.pinv);
     const uint64_t *pb = (const uint64_t *)(smb + L.pb);
     double mx = -1e300;
+    bool low = false;
     for (int g = lane; g < A.G; g += 32) {
         const double2 P = pinv[g];
-        // |P| <= 2^256: its square stays in range
-        const double n2 = CPLX ? fma(P.x, P.x, P.y * P.y) : 0.0;
+        // |P| <= 2^256, and at least 2^-400 or (INV) not used below kProdMin: its square stays in range
+        const double n2 = CPLX ? fma(P.x, P.x, P.y * P.y) : P.x * P.x;
+        if (INV) low = low || !(n2 >= kProdMin * kProdMin);
         lp[g] += CPLX ? 0.5 * log(n2) : log(P.x);
         ag[g] = apply_marshall(ag[g] + (CPLX ? atan2(P.y, P.x) : 0.0), pb[g], A.n_inner, A.inner_mask);
         if (INV) pinv[g] = CPLX ? make_double2(P.x / n2, -P.y / n2) : make_double2(1.0 / P.x, 0.0);
         mx = fmax(mx, lp[g]);
     }
+    if (INV) *small = __any_sync(0xffffffffu, low);
     mx = warp_max(mx);
     double sr = 0.0, si = 0.0;
     for (int g = lane; g < A.G; g += 32) {
@@ -343,13 +369,15 @@ __global__ void k_sym_energy(DevAmp A, DevHam H, const uint64_t *__restrict__ bi
     bool ok = true;
     for (int k = tid; k < rows; k += blockDim.x) ok = ok && range_ok[k] != 0;
     ok = __syncthreads_and(ok);
-    if (b == 0 && tid == 0) *done = ok;
-    if (!ok) return;                                         // run by k_local_generic
+    if (!ok) {                                               // run by k_local_generic
+        if (tid == 0) done[b] = 0;
+        return;
+    }
     const SymSmem L = sym_smem(G, N, M, nm, NW, true);
     unsigned char *inv = smb + L.inv;
     unsigned short *list = (unsigned short *)(smb + L.list);
     double *num = (double *)(smb + L.num);
-    __shared__ int s_n, s_sum1, s_sum2;
+    __shared__ int s_n, s_sum1, s_sum2, s_small;
     __shared__ double s_psi0;
     const uint64_t s = bits[b];
     const bool tfim = H.kind == NQS_HAM_TFIM;
@@ -394,13 +422,19 @@ __global__ void k_sym_energy(DevAmp A, DevHam H, const uint64_t *__restrict__ bi
     double2 *w = (double2 *)(smb + L.w);
     if (warp == 0) {
         double2 sum;
-        sym_weights<true, CPLX>(A, smb, L, sum);
-        if (lane == 0) s_psi0 = sum.x;
+        bool small;
+        sym_weights<true, CPLX>(A, smb, L, sum, &small);
+        if (lane == 0) {
+            s_psi0 = sum.x;
+            s_small = small;
+            done[b] = !small;
+        }
         const double2 *pinv = (const double2 *)(smb + L.pinv);
         __syncwarp();
         for (int g = lane; g < G; g += 32) w[g] = cmul(w[g], pinv[g]);
     }
     __syncthreads();
+    if (s_small) return;
     const int n = s_n;
     auto sites = [&](int m, int &u, int &v) {
         if (tfim) {
@@ -580,15 +614,15 @@ bool sym_energy_capable(const DevAmp &A, const DevHam &H) {
     return sym_base(A) && sym_smem(A.G, A.a.N, A.a.M, nm, 8, true).total <= kMaxSymSmem;
 }
 
-// Local energies of the configurations; *done (device) is 0 when weights out of range left them to
-// k_local_generic.
+// Local energies of the configurations; done[b] (device) is 0 where weights out of range or a small product
+// left one to k_local_generic.
 bool launch_sym_energy(const DevAmp &A, const DevHam &H, const uint64_t *bits, int B, double *Er, double *Ei,
                        int **done) {
     static DevBuf<double> tab;
     static DevBuf<int> flags;
     const int N = A.a.N, M = A.a.M, rows = pair_rows(N), nm = H.kind == NQS_HAM_TFIM ? H.N : H.nb1 + H.nb2;
     const bool cx = A.a.kind == KIND_CRBM;
-    if (!tab.ensure((size_t)rows * (M + 1) * (cx ? 4 : 2)) || !flags.ensure(rows + 1)) return false;
+    if (!tab.ensure((size_t)rows * (M + 1) * (cx ? 4 : 2)) || !flags.ensure((size_t)rows + B)) return false;
     cudaStream_t st = ctx().stream;
     *done = flags.p + rows;
     {
