@@ -240,7 +240,10 @@ __device__ __forceinline__ void move_sites(const DevHam &H, int m, int &u, int &
 // im each) and in column M the same of the visible biases.  range_ok[m] says that the products of
 // the row stay within the range of a double: sum_h |Re D_h| <= 350, and the factors are at most
 // 2 exp|Re D_h| (M <= 256), so nothing exceeds 2^256 e^350 < 1e230.
-constexpr double kFlipRange = 350.0;
+// Nor does a product that matters underflow while |prod (1 + r_h)| is at least kProdMin: a partial
+// product below 1e-308 times the others' 2^256 e^350 at most is 1e-19 of it.  (Hidden biases near i pi / 2, where
+// cosh acts as i sinh, take it to 0.03^M and below: such samples go through the logarithms.)
+constexpr double kFlipRange = 350.0, kProdMin = 1e-60;
 template <bool CPLX>
 __global__ void __launch_bounds__(128) k_flip_tables(DevAnsatz a, DevHam H, int nm, double *tab, int *range_ok) {
     const int lane = threadIdx.x & 31, m = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -357,6 +360,7 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
         if (CPLX) P = cmul(P, make_double2(x, __shfl_xor_sync(0xffffffffu, P.y, o)));
         else P.x *= x;
     }
+    const bool logs = !((CPLX ? fmax(fabs(P.x), fabs(P.y)) : P.x) >= kProdMin);    // true for NaN too
     // 1 / P (scaled: |P| <= 2^256)
     if (CPLX) {
         const double big = fmax(fabs(P.x), fabs(P.y)), x = P.x / big, y = P.y / big, d = big * fma(x, x, y * y);
@@ -374,7 +378,7 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
         if (m < nm) move_sites(H, m, u, v);
         const int su = (int)((s >> u) & 1ull);
         const bool anti = m < nm && (tfim || su != (int)((s >> v) & 1ull));
-        const bool ok = anti && range_ok[m] != 0;
+        const bool ok = anti && !logs && range_ok[m] != 0;
         const uint32_t am = __ballot_sync(0xffffffffu, anti);
         if (!tfim) {
             const uint32_t in = __ballot_sync(0xffffffffu, m < nm), g1 = __ballot_sync(0xffffffffu, m < H.nb1);
@@ -474,7 +478,7 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
         for (int m = 0; m < nm; m++) {
             int u, v;
             move_sites(H, m, u, v);
-            if (range_ok[m] || (!tfim && (((s >> u) ^ (s >> v)) & 1ull) == 0)) continue;
+            if ((!logs && range_ok[m]) || (!tfim && (((s >> u) ^ (s >> v)) & 1ull) == 0)) continue;
             double r, q;
             log_ratio(A, s, s ^ (1ull << u) ^ (v >= 0 ? 1ull << v : 0ull), r, q);
             const double cf = m < H.nb1 || tfim ? c1 : c2;

@@ -1,5 +1,5 @@
 """Complex RBM whose hidden units stand near their nodes (hidden biases i pi / 2: cosh acts as i sinh), so that
-the product of their |1 + exp(-2 theta)| falls to 1e-370, under a symmetry projection.  The reference
+the product of their |1 + exp(-2 theta)| falls to 1e-370, with and without a symmetry projection.  The reference
 is the definition in extended precision (long double); gradients against the oracle's sums of logarithms."""
 import numpy as np
 import pytest
@@ -57,3 +57,21 @@ def test_projected(nqs, M):
         for x, y in ((g, og), (c[0], oc[0]), (c[1], oc[1])):
             assert np.max(np.abs(x[k] - y[k])) < 1e-8 * max(np.max(np.abs(y[k])), 1.0)
     assert seen > 8
+
+
+@pytest.mark.parametrize("M", [12, 64, 144, 256])
+def test_unprojected(nqs, M):
+    cfg, a = ansatz(nqs, M)
+    ext = Extended(O.OR_CRBM, 12, M, a.params.copy(), np.arange(12)[None, :], np.ones(1, np.longdouble))
+    spins = configurations(40, M)
+    re, im = nqs.local_energy_batch(cfg, 2, 2, spins, a.log_amp_fn, a.user, complex_out=True)
+    for k, s in enumerate(spins):
+        l0, want, den = ext.log_psi(s)[0], 0.0, 1.0
+        for u, v in O.bonds(O.ham(6, 2, 2, kagome_pbc=1)):
+            want += np.longdouble(s[u] * s[v]) / 4
+            if s[u] != s[v]:
+                t = s.copy()
+                t[u], t[v] = -t[u], -t[v]
+                x = np.exp(ext.log_psi(t)[0] - l0) / 2
+                want, den = want + x, den + abs(x)
+        assert abs(re[k] + 1j * im[k] - complex(want)) < 5e-12 * den
