@@ -939,7 +939,7 @@ static bool launch_prod(const DevAmp &A, const DevHam &H, const uint64_t *bits, 
     const int nm = num_moves(H), M = A.a.M;
     if (!g_flip.ensure((size_t)(nm + 1) * (M + 1) * (C ? 4 : 2)) || !g_flip_ok.ensure((size_t)nm + 1)) return false;
     cudaStream_t st = ctx().stream;
-    {
+    if (nm > 0) {                                          // (a single site has no bonds)
         NQS_LAUNCH("flip_tables");
         k_flip_tables<C><<<(nm + 3) / 4, 128, 0, st>>>(A.a, H, nm, g_flip.p, g_flip_ok.p);
     }

@@ -611,7 +611,7 @@ bool launch_sym_gradient(const DevAmp &A, const uint64_t *bits, int B, int mode,
 
 bool sym_energy_capable(const DevAmp &A, const DevHam &H) {
     const int nm = H.kind == NQS_HAM_TFIM ? H.N : H.nb1 + H.nb2;
-    return sym_base(A) && sym_smem(A.G, A.a.N, A.a.M, nm, 8, true).total <= kMaxSymSmem;
+    return sym_base(A) && nm > 0 && sym_smem(A.G, A.a.N, A.a.M, nm, 8, true).total <= kMaxSymSmem;
 }
 
 // Local energies of the configurations; done[b] (device) is 0 where weights out of range or a small product
