@@ -894,6 +894,11 @@ int lanczos_kagome(int Lx, int Ly, double J, int pbc, const int *perm, const dou
                NQS_CUDA(cudaEventRecord(rb.done[k & 1], st));
     };
     const bool ahead = dim <= ED_SMALL_DIM;
+    // the iteration ahead is through before any return (its copies go to the pinned pair)
+    struct Drain {
+        cudaStream_t st;
+        ~Drain() { cudaStreamSynchronize(st); }
+    } drain{st};
     if (!iterate(0)) return -1;
     for (int k = 0; k < max_iters; k++) {
         if (ahead && k + 1 < max_iters) {
