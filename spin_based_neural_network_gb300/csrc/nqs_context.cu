@@ -21,6 +21,7 @@ void clear_error() { g_err[0] = 0; }
 
 bool cuda_ok(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return true;
+    cudaGetLastError();                  // reported here: not by the next launch check as well
     set_error("CUDA error %s (%d) in %s", cudaGetErrorString(e), (int)e, what);
     return false;
 }
