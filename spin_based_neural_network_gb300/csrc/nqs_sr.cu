@@ -1218,12 +1218,21 @@ static int sr_step_impl(const StepIn &in, nqs_sr_step_info_t *info, double *out_
          !NQS_CUDA(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming)) ||
          !NQS_CUDA(cudaEventCreateWithFlags(&stats_done, cudaEventDisableTiming))))
         return -1;
+    // no return leaves the statistics running beside a later call: the stream is waited for unless the
+    // solve's kernels, which start behind stats_done, are through
+    struct Leftover {
+        cudaStream_t st = nullptr;
+        ~Leftover() {
+            if (st) cudaStreamSynchronize(st);
+        }
+    } leftover;
     {
         const int chains = in.sampler ? nqs_sampler_num_chains((nqs_sampler_t *)in.sampler) : 0;
         if (!ensure_energy_scratch(w.es, Ns)) return -1;
         if (aside) {
             if (!NQS_CUDA(cudaEventRecord(forked, st)) || !NQS_CUDA(cudaStreamWaitEvent(side, forked, 0))) return -1;
             c.stream = side;
+            leftover.st = side;
         }
         const bool enqueued = enqueue_energy_stats(w.E.p, Ns, chains, w.scal.p, w.eps.p, w.es.p);
         c.stream = st;
@@ -1285,10 +1294,9 @@ static int sr_step_impl(const StepIn &in, nqs_sr_step_info_t *info, double *out_
             };
             if (!minsr_mixed_solve(w.O.p, w.gm.p, w.eps.p, rows, P, shift, c.opts.refine_sweeps,
                                    c.opts.gram_passes, c.opts.mixed_space, w.y.p, w.delta.p, &have_delta,
-                                   &resid, &f32, after, aside ? stats_done : nullptr)) {
-                if (aside) NQS_CUDA(cudaStreamSynchronize(side));   // nothing of this step is left running
+                                   &resid, &f32, after, aside ? stats_done : nullptr))
                 return -1;
-            }
+            leftover.st = nullptr;
             ss.refine_residual = resid;
             if (f32 < 0) {
                 solved = true;

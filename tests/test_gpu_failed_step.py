@@ -1,5 +1,5 @@
-"""A mixed step that fails (its 200000 x 200000 system does not fit) leaves the following step as it would be
-without it."""
+"""A mixed step that fails behind the fork of its energy statistics (its 200000 x 200000 system does not fit) leaves
+the following step on the same buffers as it would be without it."""
 import numpy as np
 import pytest
 
@@ -28,7 +28,8 @@ def test_step_after_a_failed_mixed_step():
         return np.array(E), a.params.copy()
 
     E0, p0 = step(spins[:1000])
-    with pytest.raises(nqs.NqsError):
-        step(spins, precision=abi.PREC_MIXED)
-    E, p = step(spins[:1000])
-    assert np.array_equal(E, E0) and np.array_equal(p, p0)
+    for _ in range(4):
+        with pytest.raises(nqs.NqsError):
+            step(spins, precision=abi.PREC_MIXED)
+        E, p = step(spins[:1000])
+        assert np.array_equal(E, E0) and np.array_equal(p, p0)
