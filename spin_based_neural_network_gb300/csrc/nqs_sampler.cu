@@ -23,6 +23,13 @@
 
 namespace nqs {
 
+// Factors of the FP64 Philox chains' moves, the moves in range, the chains run with them.
+struct ChainTables {
+    DevBuf<double> tab;
+    DevBuf<int> range_ok;
+    DevBuf<unsigned char> done;
+};
+
 struct Sampler {
     int N = 0, C = 1;
     nqs_config_t cfg{};
@@ -36,6 +43,7 @@ struct Sampler {
     DevBuf<int> d_bonds, d_spins;
     int nb = 0;
     int *h_current = nullptr;        // pinned, N ints (next/current)
+    ChainTables tables;              // the sampler's own: samplers may run from several host threads
     Made *made = nullptr;            // learned proposal (optional)
 };
 
@@ -1092,7 +1100,7 @@ static void launch_rbm32(dim3 grid, dim3 block, cudaStream_t st, const SampleArg
 }
 
 template <int RNG, int MOVE>
-static bool dispatch(const SampleArgs &S, const DevAmp &A, bool f32, const DevMade &md, size_t smem) {
+static bool dispatch(const SampleArgs &S, const DevAmp &A, bool f32, const DevMade &md, size_t smem, ChainTables &T) {
     dim3 grid((S.C + kSW - 1) / kSW), block(32 * kSW);
     cudaStream_t st = ctx().stream;
     const bool fused = A.G == 0 && (A.a.kind == KIND_RBM || A.a.kind == KIND_CRBM);
@@ -1122,28 +1130,25 @@ static bool dispatch(const SampleArgs &S, const DevAmp &A, bool f32, const DevMa
     const unsigned char *done = nullptr;
     if (fused && RNG == NQS_GPU_RNG_PHILOX && (MOVE != NQS_GPU_MOVE_EXCHANGE || S.nb > 0)) {
         // the chains within the product form's range; the rest by the kernel below
-        static DevBuf<double> tab;
-        static DevBuf<int> range_ok;
-        static DevBuf<unsigned char> g_done;
         const int J = (A.a.M + 31) / 32, M = A.a.M, nm = MOVE == NQS_GPU_MOVE_EXCHANGE ? S.nb : S.N;
         const bool cx = A.a.kind == KIND_CRBM;
-        if (!tab.ensure((size_t)(nm + 1) * (M + 1) * (cx ? 4 : 2)) || !range_ok.ensure(nm + 1) || !g_done.ensure(S.C))
+        if (!T.tab.ensure((size_t)(nm + 1) * (M + 1) * (cx ? 4 : 2)) || !T.range_ok.ensure(nm + 1) || !T.done.ensure(S.C))
             return false;
         {
             NQS_LAUNCH("chain_tables");
-            if (cx) k_chain_tables<true><<<(nm + 3) / 4, 128, 0, st>>>(S, A.a, MOVE, nm, tab.p, range_ok.p);
-            else k_chain_tables<false><<<(nm + 3) / 4, 128, 0, st>>>(S, A.a, MOVE, nm, tab.p, range_ok.p);
+            if (cx) k_chain_tables<true><<<(nm + 3) / 4, 128, 0, st>>>(S, A.a, MOVE, nm, T.tab.p, T.range_ok.p);
+            else k_chain_tables<false><<<(nm + 3) / 4, 128, 0, st>>>(S, A.a, MOVE, nm, T.tab.p, T.range_ok.p);
         }
         NQS_LAUNCH("sampler_ratio");
         if (M <= 16 && MOVE == NQS_GPU_MOVE_SINGLE_FLIP) {
             const size_t rs = sizeof(double) * (size_t)nm * (M + 1) * (cx ? 4 : 2);   // at most 35 KB
-            if (cx) k_sample_rbm_pair<true><<<grid, block, rs, st>>>(S, A, tab.p, range_ok.p, nm, g_done.p);
-            else k_sample_rbm_pair<false><<<grid, block, rs, st>>>(S, A, tab.p, range_ok.p, nm, g_done.p);
+            if (cx) k_sample_rbm_pair<true><<<grid, block, rs, st>>>(S, A, T.tab.p, T.range_ok.p, nm, T.done.p);
+            else k_sample_rbm_pair<false><<<grid, block, rs, st>>>(S, A, T.tab.p, T.range_ok.p, nm, T.done.p);
         } else
 #define NQS_PCASE(JJ)                                                                                              \
     case JJ:                                                                                                       \
-        if (cx) k_sample_rbm_ratio<JJ, true, MOVE><<<grid, block, 0, st>>>(S, A, tab.p, range_ok.p, nm, g_done.p); \
-        else k_sample_rbm_ratio<JJ, false, MOVE><<<grid, block, 0, st>>>(S, A, tab.p, range_ok.p, nm, g_done.p);   \
+        if (cx) k_sample_rbm_ratio<JJ, true, MOVE><<<grid, block, 0, st>>>(S, A, T.tab.p, T.range_ok.p, nm, T.done.p); \
+        else k_sample_rbm_ratio<JJ, false, MOVE><<<grid, block, 0, st>>>(S, A, T.tab.p, T.range_ok.p, nm, T.done.p);   \
         break;
         switch (J <= 4 ? J : (J + 1) / 2 * 2) {
             NQS_PCASE(1) NQS_PCASE(2) NQS_PCASE(3) NQS_PCASE(4) NQS_PCASE(6) NQS_PCASE(8)
@@ -1152,7 +1157,7 @@ static bool dispatch(const SampleArgs &S, const DevAmp &A, bool f32, const DevMa
                 return false;
         }
 #undef NQS_PCASE
-        done = g_done.p;
+        done = T.done.p;
     }
     if (fused && RNG == NQS_GPU_RNG_XORSHIFT_COMPAT) {
         int J = (A.a.M + 31) / 32;
@@ -1213,11 +1218,11 @@ bool sampler_run(Sampler *sm, int skip, int n_out, uint64_t *out, unsigned long 
         smem = made_chain_smem(sm->made, kSW);
     }
     if (sm->opts.rng == NQS_GPU_RNG_XORSHIFT_COMPAT)
-        ok = dispatch<NQS_GPU_RNG_XORSHIFT_COMPAT, NQS_GPU_MOVE_SINGLE_FLIP>(S, A, false, md, 0);
+        ok = dispatch<NQS_GPU_RNG_XORSHIFT_COMPAT, NQS_GPU_MOVE_SINGLE_FLIP>(S, A, false, md, 0, sm->tables);
     else if (sm->opts.move == NQS_GPU_MOVE_EXCHANGE)
-        ok = dispatch<NQS_GPU_RNG_PHILOX, NQS_GPU_MOVE_EXCHANGE>(S, A, f32, md, smem);
+        ok = dispatch<NQS_GPU_RNG_PHILOX, NQS_GPU_MOVE_EXCHANGE>(S, A, f32, md, smem, sm->tables);
     else
-        ok = dispatch<NQS_GPU_RNG_PHILOX, NQS_GPU_MOVE_SINGLE_FLIP>(S, A, f32, md, smem);
+        ok = dispatch<NQS_GPU_RNG_PHILOX, NQS_GPU_MOVE_SINGLE_FLIP>(S, A, f32, md, smem, sm->tables);
     sm->move_counter += (uint64_t)S.total;
     return ok;
 }
