@@ -138,7 +138,7 @@ static bool enqueue_front(BatchInst &b, cudaStream_t st) {
     uint64_t *bits = nullptr;
     if (!ansatz_refresh_derived(b.a) || !sampler_produce_dev(b.s, b.Ns, &bits, b.move.p) ||
         !launch_local_estimator(b.A, b.H, bits, b.Ns, b.E.p, b.Ei.p, b.O.p, nullptr, 1, true) ||
-        !enqueue_energy_stats(b.E.p, b.Ns, b.C, b.scal.p, b.eps.p, b.es.p) ||
+        !enqueue_energy_stats(b.E.p, b.Ns, b.C, b.scal.p, b.eps.p, b.es.p, ctx().stream) ||
         !enqueue_col_means(b.O.p, b.Ns, b.P, b.scal.p, b.gm.p, b.part.p))
         return false;
     mixed_sys_front(b.mx, st, true);

@@ -300,7 +300,8 @@ bool mixed_batch_launch(MixedBatch *b, cudaStream_t st);
 // blocks; scratch holds energy_scratch_doubles(Ns) doubles, zero before its
 // first use (its tickets return to zero after each call).
 size_t energy_scratch_doubles(int Ns);
-bool enqueue_energy_stats(const double *E, int Ns, int chains, double *scal, double *eps, double *scratch);
+bool enqueue_energy_stats(const double *E, int Ns, int chains, double *scal, double *eps, double *scratch,
+                          cudaStream_t st);
 bool enqueue_col_means(const double *O, int Ns, long P, const double *scal, double *gm, double *part);
 long col_stats_scratch(int Ns, long P);
 bool enqueue_col_dot(const double *O, int Ns, long P, const double *y, double scale, double *out);

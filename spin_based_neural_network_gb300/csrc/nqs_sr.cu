@@ -847,8 +847,8 @@ static bool ensure_energy_scratch(DevBuf<double> &b, int Ns) {
     return true;
 }
 
-bool enqueue_energy_stats(const double *E, int Ns, int chains, double *scal, double *eps, double *scratch) {
-    cudaStream_t st = ctx().stream;
+bool enqueue_energy_stats(const double *E, int Ns, int chains, double *scal, double *eps, double *scratch,
+                          cudaStream_t st) {
     const int G = es_blocks(Ns);
     unsigned *tickets = (unsigned *)scratch;
     double *part = scratch + 2, *gpart = part + (size_t)G * 4;
@@ -1231,15 +1231,14 @@ static int sr_step_impl(const StepIn &in, nqs_sr_step_info_t *info, double *out_
         if (!ensure_energy_scratch(w.es, Ns)) return -1;
         if (aside) {
             if (!NQS_CUDA(cudaEventRecord(forked, st)) || !NQS_CUDA(cudaStreamWaitEvent(side, forked, 0))) return -1;
-            c.stream = side;
             leftover.st = side;
         }
-        const bool enqueued = enqueue_energy_stats(w.E.p, Ns, chains, w.scal.p, w.eps.p, w.es.p);
-        c.stream = st;
-        if (!enqueued || (aside && !NQS_CUDA(cudaEventRecord(stats_done, side)))) return -1;
+        if (!enqueue_energy_stats(w.E.p, Ns, chains, w.scal.p, w.eps.p, w.es.p, aside ? side : st) ||
+            (aside && !NQS_CUDA(cudaEventRecord(stats_done, side))))
+            return -1;
         // <E_im> for the holomorphic force
         if (holo && (!ensure_energy_scratch(w.es2, Ns) ||
-                     !enqueue_energy_stats(w.Ei.p, Ns, 0, w.scal2.p, eps2, w.es2.p)))
+                     !enqueue_energy_stats(w.Ei.p, Ns, 0, w.scal2.p, eps2, w.es2.p, st)))
             return -1;
         // excited-state SR: the physical statistics stay in scal for the step info; the force
         // takes the augmented local energies and means
@@ -1450,7 +1449,7 @@ int nqs_gpu_ess(const double *energies, int num_samples, int num_chains, double 
     double hs[16];
     if (!NQS_CUDA(cudaMemcpyAsync(dE.p, energies, sizeof(double) * num_samples, cudaMemcpyHostToDevice, st)))
         return -1;
-    if (!enqueue_energy_stats(dE.p, num_samples, num_chains, dscal.p, deps.p, des.p) ||
+    if (!enqueue_energy_stats(dE.p, num_samples, num_chains, dscal.p, deps.p, des.p, ctx().stream) ||
         !NQS_CUDA(cudaGetLastError()) ||
         !NQS_CUDA(cudaMemcpyAsync(hs, dscal.p, sizeof(hs), cudaMemcpyDeviceToHost, st)) ||
         !NQS_CUDA(cudaStreamSynchronize(st)))

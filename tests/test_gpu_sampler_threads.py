@@ -39,3 +39,32 @@ def test_threads():
         t.join()
     for x, y in zip(alone, together):
         assert len(y) == 40 and all(np.array_equal(p, q) for p, q in zip(x, y))
+
+
+def test_beside_mixed_steps():
+    import spin_based_neural_network_gb300 as pkg
+    pkg.build()
+    from spin_based_neural_network_gb300 import abi, nqs
+    cfg = abi.config_defaults(ansatz=O.OR_CRBM, rbm_hidden_units=16, rbm_init_scale=0.1, rng_seed=5, num_decorrelate=3,
+                              num_thermalize=10, hamiltonian=abi.HAM_HEISENBERG, sr_diag_shift=1e-3, learning_rate=0.0)
+    spins = np.where(np.random.default_rng(5).random((512, 16)) < 0.5, 1, -1).astype(np.int32)
+    a, b = nqs.Ansatz(cfg, 16), nqs.Ansatz(cfg, 16)
+    nqs.set_options(precision=abi.PREC_MIXED)
+    try:
+        def step():
+            return nqs.sr_step_batch(cfg, 4, 4, a, spins)[1]
+
+        def sampler():
+            return nqs.Sampler(16, cfg, b.log_amp_fn, b.user, nqs.options(num_chains=64, rng=abi.RNG_PHILOX))
+
+        E, s, t = [step(), step()], sampler(), sampler()      # the steps' graph is captured before the threads run
+        alone, together = [s.batch(256) for _ in range(60)], [t.batch(256)]
+        thread = threading.Thread(target=lambda: together.extend(t.batch(256) for _ in range(59)))
+        thread.start()
+        while thread.is_alive():
+            E.append(step())
+        thread.join()
+    finally:
+        nqs.set_options()
+    assert all(np.array_equal(x, y) for x, y in zip(alone, together)) and len(together) == 60
+    assert all(np.array_equal(x, E[0]) for x in E)
