@@ -150,12 +150,22 @@ __device__ __forceinline__ void run_chain(const SampleArgs &S, int c, uint64_t &
 
 constexpr int kSW = 4;   // warps (chains) per block
 
+// log|psi(s') / psi(s)| from both whole amplitudes.
+__device__ __noinline__ double amplitude_log_ratio(const DevAnsatz &a, uint64_t s, int u, int v) {
+    double l0, l1, g;
+    warp_base_eval(a, s, l0, g, nullptr);
+    warp_base_eval(a, s ^ (1ull << u) ^ (v >= 0 ? 1ull << v : 0ull), l1, g, nullptr);
+    return l1 - l0;
+}
+
+// The compat chain, and the Philox chains out of the product form's range (below).  A Philox chain whose parameters
+// are not finite takes both whole amplitudes, as upstream: clogcosh gives NaN a value there.
 template <int J, bool CPLX, int RNG, int MOVE>
-__global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A) {
+__global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A, const unsigned char *done) {
     if (S.move_dev) S.move0 = *S.move_dev;
     const int lane = threadIdx.x & 31;
     const int c = blockIdx.x * kSW + (threadIdx.x >> 5);
-    if (c >= S.C) return;
+    if (c >= S.C || (done && done[c])) return;          // done: run by k_sample_rbm_ratio or _pair
     const DevAnsatz &a = A.a;
     const int M = a.M;
     const double *aR = a.p;
@@ -170,10 +180,18 @@ __global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A)
             lr[j] = CPLX ? rlogcosh(thr[j], thi[j]) : logcosh_r(thr[j]);
         }
     }
+    bool whole = false;
+    if (RNG == NQS_GPU_RNG_PHILOX) {
+#pragma unroll
+        for (int j = 0; j < J; j++) whole = whole || !isfinite(lr[j]);
+        for (int i = lane; i < a.N; i += 32) whole = whole || !isfinite(aR[i]);
+        whole = __any_sync(0xffffffffu, whole);
+    }
     auto eval = [&](int u, int v) -> double {
         const double su = (double)spin_of(s, u);
         const double sv = v >= 0 ? (double)spin_of(s, v) : 0.0;
         double d = 0.0;
+        if (RNG == NQS_GPU_RNG_PHILOX && whole) return amplitude_log_ratio(a, s, u, v);
 #pragma unroll
         for (int j = 0; j < J; j++) {
             int h = lane + 32 * j;
@@ -242,7 +260,7 @@ __global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A)
 // Range: chains whose weights could drive r_h, g_h, |1 + r_h|^2 or K out of a double's range (that need
 // |theta_h| <= 300, or 150 if complex, for every configuration, and |2 Re D_h| <= 700 for every unit and
 // |sum Re D + visible| <= 250 of every move) or are not finite leave done[c] = 0 and are run by
-// k_sample_generic, through log|psi|.
+// k_sample_rbm, through log cosh of every unit.
 constexpr float kThetaRange = 300.f;
 constexpr double kMoveRange = 250.0, kFactorRange = 700.0;
 
@@ -896,12 +914,12 @@ __global__ void __launch_bounds__(32 * kSW) k_sample_rbm32(SampleArgs S, DevAmp 
 // Any other program (symmetry projection, mean field, MLP): full evaluation of
 // every proposal, as upstream.
 template <int RNG, int MOVE>
-__global__ void __launch_bounds__(32 * kSW) k_sample_generic(SampleArgs S, DevAmp A, const unsigned char *done) {
+__global__ void __launch_bounds__(32 * kSW) k_sample_generic(SampleArgs S, DevAmp A) {
     if (S.move_dev) S.move0 = *S.move_dev;
     extern __shared__ double sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = blockIdx.x * kSW + warp;
-    if (c >= S.C || (done && done[c])) return;          // done: run by k_sample_rbm_ratio
+    if (c >= S.C) return;
     double *scr = sm + warp * 4 * (A.a.M ? A.a.M : 1);
     uint64_t s = S.bits[c];
     double la, ar, nla = 0.0;
@@ -1159,14 +1177,14 @@ static bool dispatch(const SampleArgs &S, const DevAmp &A, bool f32, const DevMa
 #undef NQS_PCASE
         done = T.done.p;
     }
-    if (fused && RNG == NQS_GPU_RNG_XORSHIFT_COMPAT) {
+    if (fused) {
         int J = (A.a.M + 31) / 32;
         bool cx = A.a.kind == KIND_CRBM;
         NQS_LAUNCH("sampler");
-#define NQS_SCASE(JJ)                                                                                        \
-    case JJ:                                                                                                 \
-        if (cx) k_sample_rbm<JJ, true, NQS_GPU_RNG_XORSHIFT_COMPAT, MOVE><<<grid, block, 0, st>>>(S, A);     \
-        else k_sample_rbm<JJ, false, NQS_GPU_RNG_XORSHIFT_COMPAT, MOVE><<<grid, block, 0, st>>>(S, A);       \
+#define NQS_SCASE(JJ)                                                                   \
+    case JJ:                                                                            \
+        if (cx) k_sample_rbm<JJ, true, RNG, MOVE><<<grid, block, 0, st>>>(S, A, done);  \
+        else k_sample_rbm<JJ, false, RNG, MOVE><<<grid, block, 0, st>>>(S, A, done);    \
         break;
         switch (J) {
             NQS_SCASE(1) NQS_SCASE(2) NQS_SCASE(3) NQS_SCASE(4) NQS_SCASE(5) NQS_SCASE(6) NQS_SCASE(7)
@@ -1179,7 +1197,7 @@ static bool dispatch(const SampleArgs &S, const DevAmp &A, bool f32, const DevMa
     } else {
         size_t smem = sizeof(double) * 4 * (A.a.M ? A.a.M : 1) * kSW;
         NQS_LAUNCH("sampler_generic");
-        k_sample_generic<RNG, MOVE><<<grid, block, smem, st>>>(S, A, done);
+        k_sample_generic<RNG, MOVE><<<grid, block, smem, st>>>(S, A);
     }
     return NQS_CUDA(cudaGetLastError());
 }
