@@ -96,7 +96,9 @@ def algorithmic_work(Ns, P, sweeps=SWEEPS):
     executes them.  gram: lower triangle incl. diagonal, N_s (N_s + 1) N_p;
     the tensor-core Gram runs it three times (hi hi^T + hi lo^T + lo hi^T) on
     the smaller system (n = min(N_s, N_p), K = the other dimension).
-    syrk: the trailing updates of the 32-wide FP64 panels, sum 2 * rest(rest+1)/2 * 32.
+    chol_solve_fp64: FP64 Cholesky n^3/3 with the forward and backward solves (2 n^2).
+    chol_syrk: the trailing updates of its 32-wide panels alone, sum 2 * rest(rest+1)/2 * 32 (the
+    allocation-free solve launches them by themselves).
     factor_refine: FP32 Cholesky n^3/3 + triangular inverse n^3/3 + per sweep
     two triangular GEMVs (2 n^2) and the FP64 residual (4 N_s N_p)."""
     gram = Ns * (Ns + 1) * P
@@ -108,7 +110,8 @@ def algorithmic_work(Ns, P, sweeps=SWEEPS):
         syrk += rest * (rest + 1) * kb
     n, k = min(Ns, P), max(Ns, P)
     fr = 2 * n ** 3 / 3 + (sweeps + 1) * (2 * n * n + 4 * Ns * P)
-    return {"gram_fp64": (gram, "fp64"), "chol_syrk": (syrk, "fp64"), "gram_tc": (3 * n * (n + 1) * k, "tensor"),
+    return {"gram_fp64": (gram, "fp64"), "chol_solve_fp64": (Ns ** 3 / 3 + 2 * Ns * Ns, "fp64"),
+            "chol_syrk": (syrk, "fp64"), "gram_tc": (3 * n * (n + 1) * k, "tensor"),
             "factor_refine": (fr, "fp32")}
 
 
@@ -330,14 +333,17 @@ NCU_TRAFFIC = {
 # taken against; these kernels do not run at that pipe's rate)
 LIMITERS = {
     "factor_refine": "latency: the chain of diagonal-block factors run by one CTA ahead of the others "
-                     "(FP32 SIMT, ~21 us per 64-wide block), then the CG operator passes (double-float "
+                     "(FP32 SIMT, ~16 us per 64-wide block), then the CG operator passes (double-float "
                      "on the FP32 pipe, L2-latency bound); the trailing and inverse tiles run on the "
                      "tensor cores beside the chain",
     "gram_tc": "tensor pipe and the TMA operand stream (TF32 hi / lo words of both row blocks per K stage, "
                "three products per stage)",
     "gram_fp64": "FP64 pipe (SIMT)",
-    "chol_syrk": "FP64 pipe (SIMT)",
+    "chol_solve_fp64": "FP64 pipes of all SMs while the trailing matrix is large; below n ~ 1000 the chain of "
+                       "panels, diagonal blocks and grid barriers",
 }
+# kernels whose roofline is reported where the step launches them
+ROOFLINES = ("gram_tc", "gram_fp64", "factor_refine", "chol_solve_fp64")
 CONV_LR0, CONV_LR1 = 0.02, 0.002   # learning-rate schedule of the accuracy run (geometric decay)
 CONV_SHIFT = 1e-4                   # its diagonal shift (the 2-D workload's)
 CONV_SWEEPS = 20                    # refinement iterations: the stacked holomorphic system is solved at shift / 4
@@ -993,8 +999,7 @@ def run_gpu(args):
     roof = roofline_of(top_name)
     kernels = {k: {"launches_per_step": v[0] / 3.0, "ms_per_step": v[1] / 3.0} for k, v in
                sorted(prof.items(), key=lambda kv: -kv[1][1])}
-    extra_roofs = {k: roofline_of(k) for k in ("gram_tc", "gram_fp64", "factor_refine", "chol_syrk")
-                   if k in prof and k != top_name}
+    extra_roofs = {k: roofline_of(k) for k in ROOFLINES if k in prof and k != top_name}
 
     # delta-theta error of the mixed step against the FP64 solve on the same samples
     delta_err = None
