@@ -33,9 +33,9 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 
 // prod (1 + r) runs down to 0.03^M and below (hidden biases near i pi / 2, where cosh acts as i sinh), past
 // the range of a double at M = 144: log-amplitudes and gradients take factors 2^512 out of it below
-// 2^-400 (e counts them), energies leave a configuration with an element below kProdMin to the logarithms.
+// 2^-400 (e counts them; tested by exponent fields after every eighth unit: |1 + r_h| is 2^-62 at least, as cos of a double), energies leave a configuration with an element below kProdMin to the logarithms.
 __device__ __forceinline__ void lift(double2 &P, int &e) {
-    if (fmax(fabs(P.x), fabs(P.y)) < 0x1p-400) {
+    if (max(__double2hiint(P.x) & 0x7fffffff, __double2hiint(P.y) & 0x7fffffff) < (1023 - 400) << 20) {
         P.x *= 0x1p512;
         P.y *= 0x1p512;
         e++;
@@ -190,7 +190,7 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
                     val[h] = make_double2(t.x * f, t.y * f);
                 }
                 P = cmul(P, d);
-                if (VALS != 1) lift(P, pe);
+                if (VALS != 1 && (j & 7) == 7) lift(P, pe);
             } else {
                 if (VALS == 1) val[h] = make_double2(e, 0.0);
                 if (VALS == 2) val[h] = make_double2((n ? em1 : -em1) / ep1, 0.0);
@@ -202,6 +202,7 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
             if (in && sl == 0) neg[j] = (unsigned char)b;
         }
     }
+    if (CPLX && VALS != 1) lift(P, pe);
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
         const double x = __shfl_xor_sync(0xffffffffu, P.x, o);
