@@ -340,9 +340,15 @@ static size_t local_prod_smem(int M, int nm) { return sizeof(double) * 4 * M + 3
 // group multiplies its lanes' products (log2 L steps; small L keeps that short, and L = 8, 16, 32
 // up to M = 64, 128, 256 bounds a lane's registers).  Lane k of a group keeps the product of the
 // group's k-th configuration, so visible factors, signs and couplings are done 32 configurations
-// at a time.
+// at a time.  theta waits in shared memory for the logarithms and the Jacobian row (a lane's registers bound the
+// warps in flight).
+// Blocks an SM asked of the compiler: five of the complex kernel with six or eight units a lane of 8 (kagome 3x3,
+// M = 54, 3001 configurations: 160 us, 180 us with the four it chooses), no bound on its registers with wider
+// groups (M = 256: 672 us, 745 us with the 128 registers it chooses), its own choice otherwise.
 template <int L, int J, bool CPLX>
-__global__ void __launch_bounds__(32 * kWarps)
+constexpr int kProdBlocks = CPLX ? (L == 8 ? (J > 4 ? 5 : 0) : 1) : 0;
+template <int L, int J, bool CPLX>
+__global__ void __launch_bounds__(32 * kWarps, kProdBlocks<L, J, CPLX>)
 k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, double *__restrict__ Er,
              double *__restrict__ Ei, double *__restrict__ O, double *__restrict__ Oi, int grad_mode,
              const double *__restrict__ tab, const int *__restrict__ range_ok, int nm, int warp_bytes) {
@@ -353,26 +359,26 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
     if (b >= B) return;
     const DevAnsatz &a = A.a;
     const int N = a.N, M = a.M;
-    double *rs = (double *)(smb + (size_t)warp * warp_bytes);      // [2 M]: r, later theta or tanh(theta)
-    double *lc = rs + 2 * M;                                        // [2 M]: log 2 cosh theta where needed
-    uint32_t *negs = (uint32_t *)(lc + 2 * M);                      // [8]: Re theta_h < 0
+    double *rs = (double *)(smb + (size_t)warp * warp_bytes);      // [2 M]: r, later log 2 cosh or tanh of theta
+    double *th = rs + 2 * M;                                        // [2 M]: theta
+    uint32_t *negs = (uint32_t *)(th + 2 * M);                      // [8]: Re theta_h < 0
     unsigned short *list = (unsigned short *)(negs + 8);            // [nm]
     const uint64_t s = bits[b];
 
-    double thr[Q], thi[Q];
     double2 P = make_double2(1.0, 0.0);                             // prod_h (1 + r_h)
 #pragma unroll
     for (int q = 0; q < Q; q++) {
         const int h = lane + 32 * q;
-        thr[q] = thi[q] = 0.0;
+        double xr = 0.0;
         if (h < M) {
-            double xr = a.p[N + h], xi = CPLX ? a.p[crbm_pr(a) + N + h] : 0.0;
+            xr = a.p[N + h];
+            double xi = CPLX ? a.p[crbm_pr(a) + N + h] : 0.0;
             for (int i = 0; i < N; i++) {
                 xr += sflip(a.wtr[(long)i * M + h], s, i);
                 if (CPLX) xi += sflip(a.wti[(long)i * M + h], s, i);
             }
-            thr[q] = xr;
-            thi[q] = xi;
+            th[h] = xr;
+            if (CPLX) th[M + h] = xi;
             const double e = exp(-2.0 * fabs(xr)) + (xr - xr);      // NaN, not 0, for an infinite theta
             if (CPLX) {
                 double sn, cs;
@@ -386,7 +392,7 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
                 P.x *= 1.0 + e;
             }
         }
-        const uint32_t neg = __ballot_sync(0xffffffffu, thr[q] < 0.0);
+        const uint32_t neg = __ballot_sync(0xffffffffu, xr < 0.0);
         if (lane == 0) negs[q] = neg;
     }
 #pragma unroll
@@ -511,21 +517,13 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
     if (CPLX) oim = warp_sum(oim);
     if (slow > 0) {                                                 // products out of range: by logarithms
         __syncwarp();
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            const int h = lane + 32 * q;
-            if (h < M) {
-                rs[h] = thr[q];
-                rs[M + h] = thi[q];
-            }
-        }
-        log_units<CPLX>(M, rs, lc);                                 // (each lane its own units)
+        log_units<CPLX>(M, th, rs);                                 // (each lane its own units)
         for (int m = 0; m < nm; m++) {
             int u, v;
             move_sites(H, m, u, v);
             if ((!logs && range_ok[m]) || (!tfim && (((s >> u) ^ (s >> v)) & 1ull) == 0)) continue;
             double r, q;
-            log_ratio<CPLX>(A, s, u, v, rs, lc, r, q);
+            log_ratio<CPLX>(A, s, u, v, th, rs, r, q);
             const double cf = m < H.nb1 || tfim ? c1 : c2;
             ore += cf * r;
             oim += cf * q;
@@ -540,15 +538,11 @@ k_local_prod(DevAmp A, DevHam H, const uint64_t *__restrict__ bits, int B, doubl
     if (grad_mode) {
         __syncwarp();
         double *tr = rs, *ti = rs + M;
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            const int h = lane + 32 * q;
-            if (h < M) {
-                if (CPLX) ctanh_d(thr[q], thi[q], tr[h], ti[h]);
-                else {
-                    tr[h] = tanh(thr[q]);
-                    ti[h] = 0.0;
-                }
+        for (int h = lane; h < M; h += 32) {
+            if (CPLX) ctanh_d(th[h], th[M + h], tr[h], ti[h]);
+            else {
+                tr[h] = tanh(th[h]);
+                ti[h] = 0.0;
             }
         }
         __syncwarp();
