@@ -525,7 +525,7 @@ __device__ int block_chol_inv64(float (*S)[BT + 1], float (*X)[BT + 1], int bs, 
 // the identity) is read once; X (zeros above the diagonal) is written to X.  Returns the
 // first non-positive pivot column below bs or -1 (the sweep goes on with a unit pivot; the
 // caller discards the block).  buf: 1024 floats.  Measured at order 8192: the owner's
-// blocks 2.94 ms a factor, as with the 16-column sweep, and the step 12.9 ms, 13.05 ms with that (this
+// blocks 2.94 ms a factor, as with the 16-column sweep, and the step 0.15 ms shorter than with that (this
 // kernel is short of registers and spills more beside the longer code).
 __device__ int block_chol_inv64_wide(const float (*S)[BT + 1], float (*X)[BT + 1], int bs, float *buf) {
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
