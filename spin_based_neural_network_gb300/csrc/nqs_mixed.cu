@@ -2949,7 +2949,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_sr(CgArgs a) {
 // [b R, b R + R) of O (and O2) there for the whole solve, and all CTAs carry p, r (and CTA 0 d) in
 // registers, E entries a thread, computed alike by every CTA.  An iteration is
 //   u_i = O_i p for the CTA's rows and their column sums sum_i O_ik u_i -> upart[b]   | grid barrier
-//   columns dealt to the CTAs: A p from the G partials and <u>                         | grid barrier
+//   columns dealt to the CTAs: A p from the partials and <u>                           | grid barrier
 //   p.Ap, the updates and r.r in every CTA,
 // two grid barriers where k_cg_sr has five and no pass over O outside shared memory.
 // What bounds it: at 256 x 288 the two barriers and the chains of dependent FP64 operations of the
@@ -2976,7 +2976,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_rows(CgArgs a, int R) {
     __shared__ double red[PS_THREADS / 32], um_s[2], quot;
     constexpr int NW = PS_THREADS / 32;
     const int G = gridDim.x, bx = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int P = (int)a.P, Ns = a.Ns, r0 = bx * R, nr = max(0, min(R, Ns - r0)), items = TWO ? 2 * nr : nr;
+    const int P = (int)a.P, Ns = a.Ns, GR = (Ns + R - 1) / R, r0 = bx * R, nr = max(0, min(R, Ns - r0)), items = TWO ? 2 * nr : nr;
     double *rows = sm, *ps = rows + (size_t)(TWO ? 2 : 1) * R * P, *us = ps + P;   // row nr + i: row i of O2
     const int S = items > 0 ? max(1, NW / items) : 1;       // warps a row
     double *up = us + 2 * R;                                // [items][S] partial row dots
@@ -3026,14 +3026,14 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_rows(CgArgs a, int R) {
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int k = tid + PS_THREADS * e;
-            if (k < P) {
+            if (k < P && nr > 0) {
                 double x = 0.0, y = 0.0;
                 for (int i = 0; i < nr; i++) x = fma(rows[(size_t)i * P + k], us[i], x);
                 for (int i = nr; i < items; i++) y = fma(rows[(size_t)i * P + k], us[i], y);
                 part[k] = TWO ? x + y : x;
             }
         }
-        if (tid < (TWO ? 2 : 1)) {
+        if (tid < (TWO ? 2 : 1) && nr > 0) {
             double v = 0.0;
             for (int i = 0; i < nr; i++) v += us[tid * nr + i];
             part[P + tid] = v;
@@ -3042,7 +3042,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_rows(CgArgs a, int R) {
         // columns bx, bx + G, ... of A p, a warp each; the last warp also forms <u>, <u2>
         if (warp == NW - 1) {
             double v = 0.0, v2 = 0.0;
-            for (int g = lane; g < G; g += 32) {
+            for (int g = lane; g < GR; g += 32) {
                 v += __ldcg(a.upart + (size_t)g * (P + 2) + P);
                 if (TWO) v2 += __ldcg(a.upart + (size_t)g * (P + 2) + P + 1);
             }
@@ -3056,7 +3056,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_cg_rows(CgArgs a, int R) {
         for (int k0 = bx + G * warp; k0 - G * warp < P; k0 += G * NW) {      // the same trip count in all warps
             double v = 0.0;
             if (k0 < P)
-                for (int g = lane; g < G; g += 32) v += __ldcg(a.upart + (size_t)g * (P + 2) + k0);
+                for (int g = lane; g < GR; g += 32) v += __ldcg(a.upart + (size_t)g * (P + 2) + k0);
             v = warp_sum(v);
             __syncthreads();                                                 // um_s
             if (lane == 0 && k0 < P) {
@@ -3141,6 +3141,9 @@ bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double 
     // rows in shared memory where they fit: at least four a CTA (fewer would only add CTAs to the
     // barriers: 256 x 288 takes the same time on 64 CTAs as on 152)
     const int R = std::max(4, (Ns + c.sm_count - 1) / c.sm_count), Gr = (Ns + R - 1) / R;
+    // and CTAs without rows for the columns of few samples, two columns a warp (5 x 1987, 9 iterations: 186 us, 2151 us
+    // on the two CTAs with rows, 698 us by k_cg_sr)
+    const int Gc = std::max(Gr, std::min(c.sm_count, (int)((P + 15) / 16)));
     const size_t rsm = cg_rows_smem(R, P, O2 != nullptr);
     const bool in_smem = P <= CG_MAX_P && rsm <= 224 * 1024;
     if (!r.ensure(P) || !p.ensure(P) || !Ap.ensure(P) || !u.ensure(Ns) ||
@@ -3172,7 +3175,7 @@ bool cg_sr_solve(const double *O, int Ns, long P, const double *F, const double 
     const double jac_bytes = 8.0 * (double)Ns * (double)P * (O2 ? 2.0 : 1.0);
     const int grid = std::max(8, std::min(c.sm_count, (int)std::ceil(jac_bytes / (256.0 * 1024.0))));
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)(in_smem ? Gr : grid));
+    lc.gridDim = dim3((unsigned)(in_smem ? Gc : grid));
     lc.blockDim = dim3(PS_THREADS);
     lc.dynamicSmemBytes = in_smem ? rsm : 0;
     lc.stream = st;
