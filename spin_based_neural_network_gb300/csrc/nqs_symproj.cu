@@ -44,6 +44,11 @@ __device__ __forceinline__ void lift(double2 &P, int &e) {
 // No product of the energies that matters in the sum underflows above it: a partial product below 1e-308 times
 // the others' 2^256 e^350 at most is 1e-19 of 1e-60.
 constexpr double kProdMin = 1e-60;
+// A sum over the group that cancels to this share of its terms is rounding (a node: an element of the other
+// sign maps the configuration to itself).  Energies leave it to the logarithms too, and amplitudes to the same sums:
+// the residues of psi(s) and of its connected configurations, nodes as well, then have finite ratios, where sums in
+// another order come out as 0 ten times as often and the ratios are infinite.
+constexpr double kNodeMin = 1e-12;
 
 __host__ __device__ inline int pair_rows(int N) { return N * (N - 1) / 2 + N; }
 // row of the pair i < j, or of the single site i (j < 0)
@@ -224,11 +229,11 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
 }
 
 // Weights w_g = chi_g exp(lp_g - max + i arg_g) by one warp, an element a lane (inner Marshall layers
-// included; INV: pinv becomes 1 / prod (1 + r), small says that one of these is below kProdMin or NaN);
-// returns max and sum_g w_g (all lanes).
+// included; INV: pinv becomes 1 / prod (1 + r)); returns max and sum_g w_g (all lanes).  out, when given, says that
+// the sum cancels to kNodeMin, or (INV) that a prod (1 + r) is below kProdMin or NaN.
 template <bool INV, bool CPLX>
 __device__ __forceinline__ double sym_weights(const DevAmp &A, unsigned char *smb, const SymSmem &L, double2 &sum,
-                                              bool *small = nullptr) {
+                                              bool *out = nullptr) {
     const int lane = threadIdx.x & 31;
     double *lp = (double *)(smb + L.lp), *ag = (double *)(smb + L.ag);
     double2 *w = (double2 *)(smb + L.w), *pinv = (double2 *)(smb + L.pinv);
@@ -245,9 +250,8 @@ __device__ __forceinline__ double sym_weights(const DevAmp &A, unsigned char *sm
         if (INV) pinv[g] = CPLX ? make_double2(P.x / n2, -P.y / n2) : make_double2(1.0 / P.x, 0.0);
         mx = fmax(mx, lp[g]);
     }
-    if (INV) *small = __any_sync(0xffffffffu, low);
     mx = warp_max(mx);
-    double sr = 0.0, si = 0.0;
+    double sr = 0.0, si = 0.0, sa = 0.0;
     for (int g = lane; g < A.G; g += 32) {
         const double m = A.chars[g] * exp(lp[g] - mx);
         double sn, cs;
@@ -255,9 +259,19 @@ __device__ __forceinline__ double sym_weights(const DevAmp &A, unsigned char *sm
         w[g] = make_double2(m * cs, m * sn);
         sr += m * cs;
         si += m * sn;
+        sa += fabs(m);
     }
     sum = make_double2(warp_sum(sr), warp_sum(si));
+    if (out) {
+        sa = warp_sum(sa);
+        *out = __any_sync(0xffffffffu, low) || !(fabs(sum.x) > kNodeMin * sa);
+    }
     return mx;
+}
+
+// A node's amplitude, by the sums of the other programs' kernels.
+__device__ __noinline__ void node_amplitude(const DevAmp &A, uint64_t s, double &la, double &ar) {
+    warp_amp_eval(A, s, la, ar, nullptr);
 }
 
 template <bool CPLX>
@@ -272,13 +286,15 @@ __global__ void k_sym_log_amp(DevAmp A, const uint64_t *__restrict__ bits, doubl
     __syncthreads();
     if (warp != 0) return;
     double2 sum;
-    const double mx = sym_weights<false, CPLX>(A, smb, L, sum), as = fabs(sum.x);
-    double l = -1e300, p = 0.0;
-    if (as > 0.0) {
-        l = log(as) + mx - 0.5 * log((double)A.G);
-        p = sum.x < 0.0 ? kPi : 0.0;
+    bool node;
+    const double mx = sym_weights<false, CPLX>(A, smb, L, sum, &node);
+    double l, p;
+    if (node) {
+        node_amplitude(A, s, l, p);
+    } else {
+        l = log(fabs(sum.x)) + mx - 0.5 * log((double)A.G);
+        p = apply_marshall(sum.x < 0.0 ? kPi : 0.0, s, A.n_outer, A.outer_mask);
     }
-    p = apply_marshall(p, s, A.n_outer, A.outer_mask);
     if ((threadIdx.x & 31) == 0) {
         if (la) la[b] = l;
         if (ar) ar[b] = p;
@@ -378,7 +394,7 @@ __global__ void k_sym_energy(DevAmp A, DevHam H, const uint64_t *__restrict__ bi
     unsigned char *inv = smb + L.inv;
     unsigned short *list = (unsigned short *)(smb + L.list);
     double *num = (double *)(smb + L.num);
-    __shared__ int s_n, s_sum1, s_sum2, s_small;
+    __shared__ int s_n, s_sum1, s_sum2, s_out;
     __shared__ double s_psi0;
     const uint64_t s = bits[b];
     const bool tfim = H.kind == NQS_HAM_TFIM;
@@ -423,19 +439,19 @@ __global__ void k_sym_energy(DevAmp A, DevHam H, const uint64_t *__restrict__ bi
     double2 *w = (double2 *)(smb + L.w);
     if (warp == 0) {
         double2 sum;
-        bool small;
-        sym_weights<true, CPLX>(A, smb, L, sum, &small);
+        bool out;
+        sym_weights<true, CPLX>(A, smb, L, sum, &out);
         if (lane == 0) {
             s_psi0 = sum.x;
-            s_small = small;
-            done[b] = !small;
+            s_out = out;
+            done[b] = !out;
         }
         const double2 *pinv = (const double2 *)(smb + L.pinv);
         __syncwarp();
         for (int g = lane; g < G; g += 32) w[g] = cmul(w[g], pinv[g]);
     }
     __syncthreads();
-    if (s_small) return;
+    if (s_out) return;
     const int n = s_n;
     auto sites = [&](int m, int &u, int &v) {
         if (tfim) {
@@ -537,7 +553,6 @@ __global__ void k_sym_energy(DevAmp A, DevHam H, const uint64_t *__restrict__ bi
     if (warp != 0) return;
     const int par0 = marshall_count(A, s);
     const double psi0 = s_psi0, c1 = tfim ? -H.Gamma : 0.5 * H.Jxy, c2 = 0.5 * H.J2;
-    const bool node = !(fabs(psi0) > 0.0);                   // zero (or NaN): ratios as of log|psi| = -1e300
     double off = 0.0;
     for (int c = lane; c < n; c += 32) {
         const int m = list[c];
@@ -547,14 +562,13 @@ __global__ void k_sym_energy(DevAmp A, DevHam H, const uint64_t *__restrict__ bi
         sites(m, u, v);
         const uint64_t s2 = s ^ (1ull << u) ^ (v >= 0 ? 1ull << v : 0ull);
         const double cf = m < H.nb1 || tfim ? c1 : c2;
-        if (node) x = fabs(x) > 0.0 ? (x > 0.0 ? INFINITY : -INFINITY) : 1.0;
         off = fma(((marshall_count(A, s2) - par0) & 1) ? -cf : cf, x, off);
     }
     off = warp_sum(off);
     if (lane == 0) {
         double diag = tfim ? -H.J * (double)s_sum1 : 0.25 * H.Jz * (double)s_sum1;
         if (H.nb2 > 0) diag += 0.25 * H.J2 * (double)s_sum2;
-        if (Er) Er[b] = diag + (node ? off : off / psi0);
+        if (Er) Er[b] = diag + off / psi0;
         if (Ei) Ei[b] = 0.0;
     }
 }
@@ -615,8 +629,8 @@ bool sym_energy_capable(const DevAmp &A, const DevHam &H) {
     return sym_base(A) && nm > 0 && sym_smem(A.G, A.a.N, A.a.M, nm, 8, true).total <= kMaxSymSmem;
 }
 
-// Local energies of the configurations; done[b] (device) is 0 where weights out of range or a small product
-// left one to k_local_generic.
+// Local energies of the configurations; done[b] (device) is 0 where weights out of range, a small product or a
+// node left one to k_local_generic.
 bool launch_sym_energy(const DevAmp &A, const DevHam &H, const uint64_t *bits, int B, double *Er, double *Ei,
                        int **done) {
     static DevBuf<double> tab;
