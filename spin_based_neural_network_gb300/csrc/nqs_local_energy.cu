@@ -217,7 +217,7 @@ __device__ void rbm_row_from_t(const DevAnsatz &a, uint64_t bits, int mode, doub
 // 16 clocks and SM, and the estimator is bound by their number.  prod 1 / (1 + r_h) is one
 // factor per sample.
 //
-// Measured: kagome 3x3, complex RBM M = 54, 3001 configurations: 185 us and 12 us for the tables,
+// Measured: kagome 3x3, complex RBM M = 54, 3001 configurations: 162 us and 12 us for the tables,
 // against 1999 us by logarithms; 4x4 Heisenberg, complex RBM M = 32, 1000 samples with Jacobian
 // rows: 45 + 12 against 339 us; 4x4 TFIM, RBM M = 16, 256 samples: 16 + 6 against 92 us.
 

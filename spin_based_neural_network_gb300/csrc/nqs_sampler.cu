@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(32 * kSW) k_sample_rbm(SampleArgs S, DevAmp A,
 // before the current move is decided.  Measured: 16 chains x 1024 proposals, 16-unit RBM: 656 us
 // against 1980 us (tanh recomputed on every accept);
 // 512 chains x 144 exchange proposals, 6x6 complex
-// RBM, 72 units: 174 us against 1161 us (log cosh of every unit).
+// RBM, 72 units: 169 us against 1161 us (log cosh of every unit).
 //
 // Range: chains whose weights could drive r_h, g_h, |1 + r_h|^2 or K out of a double's range (that need
 // |theta_h| <= 300, or 150 if complex, for every configuration, and |2 Re D_h| <= 700 for every unit and

@@ -9,9 +9,9 @@
 // product of factors of nqs_local_energy.cu, here from tables over all pairs of sites (g maps a
 // bond onto a pair).  The FP64 pipe (a warp instruction per 16 clocks and SM) bounds all of it.
 //
-// Measured (kagome 2x2, 8 elements, complex RBM M = 64, 1024 samples): local energies 290 us, complex
-// gradient 164 us; kagome 3x3, 18 elements, M = 40, 500 configurations: log-amplitudes 130 us,
-// gradient 191 us; before, with log 2 cosh of every unit of every amplitude and one warp per
+// Measured (kagome 2x2, 8 elements, complex RBM M = 64, 1024 samples): local energies 308 us, complex
+// gradient 165 us; kagome 3x3, 18 elements, M = 40, 500 configurations: log-amplitudes 133 us,
+// gradient 194 us; before, with log 2 cosh of every unit of every amplitude and one warp per
 // configuration: 3811, 625, 360 and 866 us.
 #include <math.h>
 
@@ -175,11 +175,19 @@ __device__ __forceinline__ void sym_elements(const DevAmp &A, int g0, unsigned c
                 if (CPLX) xi += sflip(a.wti[(long)i * M + h], pb, i);
             }
             const bool n = xr < 0.0;
-            // r is kept for factors X of up to exp(350), so it has to be exact to its own size: from exp; the
-            // sums 1 + r and 1 - r take it from expm1.  (NaN for an infinite theta)
-            const double em1 = VALS == 1 ? 0.0 : expm1(-2.0 * fabs(xr)) + (xr - xr);
-            const double e = VALS == 1 ? exp(-2.0 * fabs(xr)) + (xr - xr) : 1.0 + em1;
-            const double ep1 = VALS == 1 ? 1.0 + e : 2.0 + em1;
+            // r is kept for factors X of up to exp(350), so it has to be exact to its own size: from exp below 1/2,
+            // from expm1, which the sums 1 + r and 1 - r take as it is, above (with exp there too the energies at weights
+            // of 0.05 were 10 % further off; both functions cost the kernel 7 %).  (NaN for an infinite theta)
+            double em1, e;
+            if (VALS == 1 && fabs(xr) > 0.34657359) {
+                e = exp(-2.0 * fabs(xr));
+                em1 = e - 1.0;
+            } else {
+                em1 = expm1(-2.0 * fabs(xr));
+                e = 1.0 + em1;
+            }
+            em1 += xr - xr;
+            const double ep1 = 2.0 + em1;
             lr += fabs(xr);
             if (CPLX) {
                 li += n ? -xi : xi;
